@@ -346,7 +346,8 @@ void susy_b200_destroy(susy_b200_lattice* h) {
     h->U = h->Uinv = h->pd = h->U32 = h->Uinv32 = h->pd32 = nullptr, h->nbrtab = nullptr;
   void* ptrs[] = {h->U, h->mom, h->Uinv, h->force, h->det, h->pd, h->zw, h->D, h->F,
                   h->U32, h->Uinv32, h->pd32, h->stage, h->ms, h->bigpart, h->gen, h->prn,
-                  h->rng_bad, h->ptrbuf, h->nbrtab, h->meas, h->trace[0], h->trace[1]};
+                  h->rng_bad, h->ptrbuf, h->nbrtab, h->meas, h->trace[0], h->trace[1],
+                  h->ftrace};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   for (int i = 0; i < SUSY_NSCRATCH; i++) {

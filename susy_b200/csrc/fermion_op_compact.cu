@@ -84,6 +84,7 @@ int upload_fop_terms(int device, cudaStream_t st) {
   cudaMemcpyToSymbol(c_disp, tb.disp.data(), tb.disp.size() * sizeof(char4));
   cudaMemcpyToSymbol(c_slot_disp, slot_disp, sizeof(slot_disp));
   cudaMemcpyToSymbol(c_nslot, nslot, sizeof(nslot));
+  if (upload_force_terms() != 0) return -2;
   if (cudaGetLastError() != cudaSuccess) return -2;
   prefer_l1_grouped<double>();
   prefer_l1_grouped<float>();

@@ -10,10 +10,11 @@
 //   determinant force             det_force                det_force.c:6-78
 //   link update                   update_u                 update_o.c:20-35
 //   action densities              action.c:106-286
-// One thread computes the force on one link (site x, direction M): every
-// neighbour product the reference builds by gathers is formed in registers
-// from the SoA fields, with compile-time offsets.
+// The fermion force evaluates a table of products per link (32 sites of one
+// direction a block); in the other kernels one thread computes one link or
+// site, with compile-time offsets.
 #include "common.cuh"
+#include "fop_table.cuh"
 #include "kernels.h"
 
 namespace susy {
@@ -22,219 +23,281 @@ constexpr int FT = 128;
 
 struct FfArgs {
   Geo g;
-  const double2 *U, *Uinv, *pd;
+  const double2 *Uinv, *pd;
   const double2 *sol, *psol;  // psol = D sol (not yet scaled by amp)
   double2* force;             // accumulates amp * f_U^dag
+  const double2* tr;          // traces of k_ff_traces, [12][S]
+  const int* nbrtab;          // the operator's neighbour index table
   double amp, G;
   int doG;
 };
 
-// T_b(y) = Tr[U_b(y)^{-1} psi_b(y)], psi read from fld component 1+b
-template <int N, bool ADJ>
-SUSY_D Cx<double> Ttr(const FfArgs& a, const double2* fld, int b, int y) {
-  Mat<N, double> ui = ldm<N, double>(a.Uinv, b, y, a.g.S);
-  Mat<N, double> ps = ldm<N, double, ADJ>(fld, 1 + b, y, a.g.S);
-  return trace_nn(ui, ps);
+// The force on link M as a table.  Its hermitian conjugate g = f_U^dag, the
+// form the pole sum wants, is 32 products per link (the reference forms 44:
+// its F1Q of the split (DE | AB) and its F2Q of (AB | DE), update_h.c:
+// 272-462, are the same two products, since D + E + M = -(A + B), with the
+// same signs and BC factors), eight of each operand pattern:
+//   FF_SP: sol psol^dag   FF_PS: psol^dag sol
+//   FF_PD: psol sol^dag   FF_DP: sol^dag psol
+enum { FF_SP = 0, FF_PS = 1, FF_PD = 2, FF_DP = 3 };
+constexpr int FF_ROWS = 8;
+
+struct FfTerm {
+  int8_t kl, dl, kr, dr;   // components and displacement indices of the factors
+  int8_t b1, b2;           // time displacements of the two BC factors
+  int8_t pad[2];
+  float coef;
+};
+__constant__ FfTerm c_ff[NUMLINK][4][FF_ROWS];
+
+int upload_force_terms() {
+  TermBuilder tb = fop_terms();
+  const size_t nd = tb.disp.size();
+  FfTerm t[NUMLINK][4][FF_ROWS] = {};
+  int n[NUMLINK][4] = {};
+  auto add = [&](int M, int pat, double coef, int b1, int b2, int kl, int dl, int kr, int dr) {
+    if (n[M][pat] >= FF_ROWS) {
+      n[M][pat]++;
+      return;
+    }
+    FfTerm& T = t[M][pat][n[M][pat]++];
+    T.kl = (int8_t)kl; T.dl = (int8_t)dl; T.kr = (int8_t)kr; T.dr = (int8_t)dr;
+    T.b1 = (int8_t)b1; T.b2 = (int8_t)b2;
+    T.coef = (float)coef;
+  };
+  for (int M = 0; M < NUMLINK; M++) {
+    const int o = tb.dl({}), pM = tb.dl({M}), tM = et(M);
+    // S/L: half of psi_M bc eta'(x+M) - eta' psi_M - psi'_M bc eta(x+M) + eta psi'_M
+    add(M, FF_SP, 0.5, tM, 0, 1 + M, o, 0, pM);
+    add(M, FF_PS, -0.5, 0, 0, 0, o, 1 + M, o);
+    add(M, FF_PS, -0.5, tM, 0, 1 + M, o, 0, pM);
+    add(M, FF_SP, 0.5, 0, 0, 0, o, 1 + M, o);
+    // V/P
+    for (int nu = 0; nu < NUMLINK; nu++) {
+      if (nu == M) continue;
+      const double sg = M < nu ? 1.0 : -1.0;
+      const int q = 6 + pidx(M, nu), mn = tb.dl({}, {nu});
+      add(M, FF_PD, -sg, tM, 0, q, o, 1 + nu, pM);
+      add(M, FF_DP, sg, 0, 0, 1 + nu, mn, q, mn);
+      add(M, FF_DP, sg, tM, 0, q, o, 1 + nu, pM);
+      add(M, FF_PD, -sg, 0, 0, 1 + nu, mn, q, mn);
+    }
+    // Q-closed, for every split of the other four directions into (AB | DE)
+    for (int A = 0; A < NUMLINK; A++)
+      for (int B = A + 1; B < NUMLINK; B++) {
+        if (A == M || B == M) continue;
+        int K[2], k = 0;
+        for (int v = 0; v < NUMLINK; v++)
+          if (v != M && v != A && v != B) K[k++] = v;
+        const int D = K[0], E = K[1];
+        const double p = eps5(D, E, M, A, B);
+        // x + A + B + M = x - D - E
+        add(M, FF_PS, -p, et(A) + et(B) + tM, tM, 6 + pidx(D, E), tb.dl({A, B, M}),
+            6 + pidx(A, B), pM);
+        add(M, FF_SP, p, -et(A) - et(B), tM, 6 + pidx(A, B), tb.dl({}, {A, B}),
+            6 + pidx(D, E), pM);
+      }
+    for (int pat = 0; pat < 4; pat++)
+      if (n[M][pat] != FF_ROWS) return -1;
+  }
+  if (tb.disp.size() != nd) return -1;   // every displacement is one of the operator's
+  return cudaMemcpyToSymbol(c_ff, t, sizeof(t)) == cudaSuccess ? 0 : -2;
 }
 
-// detF(eta, psi, sign) contribution to f_U[M] (update_h.c:477-651);
-// ADJ_ETA/ADJ_PSI select whether eta / psi are read adjointed from psol.
-template <int N, int M, bool ETA_PSOL>
-SUSY_D void detF_term(Mat<N, double>& f, const FfArgs& a, const Site& c) {
-  const Geo& g = a.g;
-  const int S = g.S, s = c.s;
-  // sign +1: eta = psol site (adjointed), psi = sol links, localG = -G/2
-  // sign -1: eta = sol site, psi = psol links (adjointed), localG = +G/2
-  const double2* etaf = ETA_PSOL ? a.psol : a.sol;
-  const double2* psif = ETA_PSOL ? a.sol : a.psol;
-  constexpr bool AE = ETA_PSOL, AP = !ETA_PSOL;
-  const double localG = (ETA_PSOL ? -0.5 : 0.5) * a.G;
-  const Cx<double> te0 = ldtr<N, double, AE>(etaf, 0, s, S);
-  const Cx<double> TM0 = Ttr<N, AP>(a, psif, M, s);
-  const int pM = nbr(g, c, ex(M), ey(M), ez(M), et(M));
-  Cx<double> plaq(0, 0), adjt(0, 0), inv(0, 0);
-#pragma unroll
-  for (int b = 0; b < NUMLINK; b++) {
-    if (b == M) continue;
-    const int mb = nbr(g, c, -ex(b), -ey(b), -ez(b), -et(b));
-    const int pb = nbr(g, c, ex(b), ey(b), ez(b), et(b));
-    const int mbpM = nbr(g, c, ex(M) - ex(b), ey(M) - ey(b), ez(M) - ez(b), et(M) - et(b));
-    const double bcM = bcf<double>(g, c, et(M));
-    const double bcb = bcf<double>(g, c, et(b));
-    const double bcmb = bcf<double>(g, c, -et(b));
-    // bc[M] evaluated at site x - b
-    Site cm = c;
-    cm.t = wrap(c.t - et(b), g.nt);
-    const double bcM_mb = bcf<double>(g, cm, et(M));
-    const Cx<double> te_mb = ldtr<N, double, AE>(etaf, 0, mb, S);
-    const Cx<double> DbM = te0 * ldc<double>(a.pd + (size_t)(b * 5 + M) * S + s);
-    const Cx<double> DMb = te0 * ldc<double>(a.pd + (size_t)(M * 5 + b) * S + s);
-    const Cx<double> DMb_mb = te_mb * ldc<double>(a.pd + (size_t)(M * 5 + b) * S + mb);
-    const Cx<double> DbM_mb = te_mb * ldc<double>(a.pd + (size_t)(b * 5 + M) * S + mb);
-    const Cx<double> Tb0 = Ttr<N, AP>(a, psif, b, s);
-    const Cx<double> Tb_pM = Ttr<N, AP>(a, psif, b, pM);
-    const Cx<double> Tb_mb = Ttr<N, AP>(a, psif, b, mb);
-    const Cx<double> TM_pb = Ttr<N, AP>(a, psif, M, pb);
-    const Cx<double> TM_mb = Ttr<N, AP>(a, psif, M, mb);
-    const Cx<double> Tb_mbpM = Ttr<N, AP>(a, psif, b, mbpM);
-    plaq = plaq + DbM * (TM0 + bcM * Tb_pM);
-    plaq = plaq + DMb_mb * (Tb_mb + bcmb * TM0);
-    adjt = adjt + DMb * (Tb0 + bcb * TM_pb);
-    adjt = adjt + DbM_mb * (TM_mb + bcM_mb * Tb_mbpM);
-    inv = inv + DbM + bcmb * DMb_mb;
+// Every trace detF needs, once per site instead of once per link that reads
+// it (up to 20 of two matrices each per link and source before):
+//   tr[e] = Tr U_e^-1 psi_e, tr[5 + e] = Tr U_e^-1 psi'_e^dag,
+//   tr[10] = Tr eta, tr[11] = conj Tr eta'
+// (psi, eta of sol, primed of psol).  One thread per site and e = blockIdx.y;
+// e = 5 the two of the site component.
+template <int N>
+__global__ void __launch_bounds__(FT) k_ff_traces(FfArgs a, double2* tr) {
+  const int s = blockIdx.x * FT + threadIdx.x, e = blockIdx.y, S = a.g.S;
+  if (s >= a.g.V) return;
+  if (e == NUMLINK) {
+    stc<double>(tr + (size_t)10 * S + s, ldtr<N, double, false>(a.sol, 0, s, S));
+    stc<double>(tr + (size_t)11 * S + s, ldtr<N, double, true>(a.psol, 0, s, S));
+    return;
   }
-  Mat<N, double> ui = ldm<N, double>(a.Uinv, M, s, S);
-  Mat<N, double> ps = ldm<N, double, AP>(psif, 1 + M, s, S);
-  Mat<N, double> upu = mul(mul(ui, ps), ui);
-  axpy(f, localG * plaq, ui);
-  axpy(f, conj(localG * adjt), ui);
-  axpy(f, Cx<double>(-localG * inv.re, -localG * inv.im), upu);
-}
-
-// Q-closed pieces with c = M for one split of the complement into (A,B), (D,E)
-template <int N, int M, int A, int B, int D, int E>
-SUSY_D void fq_terms(Mat<N, double>& f, const FfArgs& a, const Site& c) {
-  const Geo& g = a.g;
-  const int S = g.S;
-  constexpr int abx = ex(A) + ex(B), aby = ey(A) + ey(B), abz = ez(A) + ez(B), abt = et(A) + et(B);
-  const int pM = nbr(g, c, ex(M), ey(M), ez(M), et(M));
-  const int pabM = nbr(g, c, abx + ex(M), aby + ey(M), abz + ez(M), abt + et(M));
-  const int mab = nbr(g, c, -abx, -aby, -abz, -abt);
-  const double bcM = bcf<double>(g, c, et(M));
-  const double bc3 = bcf<double>(g, c, abt + et(M));
-  const double bc2m = bcf<double>(g, c, -abt);
-  Mat<N, double> tm;
-  tm.zero();
-  // F1Q: chi'_DE(x+A+B+M) (p bc3 bc[M] chi_AB(x+M)) + (-p bc2 bc[M] chi_AB(x-A-B)) chi'_DE(x+M)
-  {
-    const double p = (double)eps5(D, E, M, A, B);
-    Mat<N, double> l0 = ldm<N, double, true>(a.psol, 6 + pidx(D, E), pabM, S);
-    Mat<N, double> l1 = ldm<N, double>(a.sol, 6 + pidx(A, B), pM, S);
-    mac<0>(tm, p * bc3 * bcM, l0, l1);
-    Mat<N, double> l3 = ldm<N, double>(a.sol, 6 + pidx(A, B), mab, S);
-    Mat<N, double> l2 = ldm<N, double, true>(a.psol, 6 + pidx(D, E), pM, S);
-    mac<0>(tm, -p * bc2m * bcM, l3, l2);
-  }
-  // F2Q: chi'_AB(x-A-B) (p bc2 bc[M] chi_DE(x+M)) + (-p bc3 bc[M] chi_DE(x+A+B+M)) chi'_AB(x+M)
-  {
-    const double p = (double)eps5(A, B, M, D, E);
-    Mat<N, double> l0 = ldm<N, double, true>(a.psol, 6 + pidx(A, B), mab, S);
-    Mat<N, double> l1 = ldm<N, double>(a.sol, 6 + pidx(D, E), pM, S);
-    mac<0>(tm, p * bc2m * bcM, l0, l1);
-    Mat<N, double> l3 = ldm<N, double>(a.sol, 6 + pidx(D, E), pabM, S);
-    Mat<N, double> l2 = ldm<N, double, true>(a.psol, 6 + pidx(A, B), pM, S);
-    mac<0>(tm, -p * bc3 * bcM, l3, l2);
-  }
-  // f_U[M] += -1/2 tm^dag
+  const double2* pu = a.Uinv + (size_t)(e * N * N) * S + s;
+  const double2* ps = a.sol + (size_t)((1 + e) * N * N) * S + s;
+  const double2* pp = a.psol + (size_t)((1 + e) * N * N) * S + s;
+  Cx<double> t0(0, 0), t1(0, 0);
 #pragma unroll
   for (int i = 0; i < N; i++)
 #pragma unroll
-    for (int j = 0; j < N; j++) {
-      f.e[i][j].re -= 0.5 * tm.e[j][i].re;
-      f.e[i][j].im += 0.5 * tm.e[j][i].im;
+    for (int k = 0; k < N; k++) {
+      const Cx<double> u = ldc<double>(pu + (size_t)(i * N + k) * S);
+      t0 = t0 + u * ldc<double>(ps + (size_t)(k * N + i) * S);
+      t1 = t1 + u * conj(ldc<double>(pp + (size_t)(i * N + k) * S));
     }
+  stc<double>(tr + (size_t)e * S + s, t0);
+  stc<double>(tr + (size_t)(5 + e) * S + s, t1);
 }
 
-template <int M>
-struct Compl4 {
-  static constexpr int k(int n) {
-    int c = 0;
-    for (int v = 0; v < 5; v++) {
-      if (v == M) continue;
-      if (c == n) return v;
-      c++;
-    }
-    return -1;
-  }
-  static constexpr int K0 = k(0), K1 = k(1), K2 = k(2), K3 = k(3);
-};
-
-template <int N, int M>
-SUSY_D Mat<N, double> fforce_out(const FfArgs& a, const Site& c) {
+// One direction b's share of detF (update_h.c:477-651), for both of its
+// calls (q = 0: eta' with psi, localG = -G/2; q = 1: eta with psi', +G/2):
+//   u   coefficient of U_M^-1: localG plaq + conj(localG adj)
+//   inv coefficient of U_M^-1 psi U_M^-1, per call
+SUSY_D void ff_det(const FfArgs& a, const Site& c, int M, int b, Cx<double>& u, Cx<double>* inv) {
   const Geo& g = a.g;
   const int S = g.S, s = c.s;
   const int pM = nbr(g, c, ex(M), ey(M), ez(M), et(M));
+  const int mb = nbr(g, c, -ex(b), -ey(b), -ez(b), -et(b));
+  const int pb = nbr(g, c, ex(b), ey(b), ez(b), et(b));
+  const int mbpM = nbr(g, c, ex(M) - ex(b), ey(M) - ey(b), ez(M) - ez(b), et(M) - et(b));
   const double bcM = bcf<double>(g, c, et(M));
-  Mat<N, double> f;
-  // S/L terms: up = psi_M bc eta'(x+M) - eta' psi_M - psi'_M bc eta(x+M) + eta psi'_M
-  {
-    Mat<N, double> up;
-    up.zero();
-    Mat<N, double> psM = ldm<N, double>(a.sol, 1 + M, s, S);
-    Mat<N, double> etp = ldm<N, double, true>(a.psol, 0, pM, S);
-    mac<0>(up, bcM, psM, etp);
-    etp = ldm<N, double, true>(a.psol, 0, s, S);
-    mac<0>(up, -1.0, etp, psM);
-    Mat<N, double> ppM = ldm<N, double, true>(a.psol, 1 + M, s, S);
-    Mat<N, double> et_ = ldm<N, double>(a.sol, 0, pM, S);
-    mac<0>(up, -bcM, ppM, et_);
-    et_ = ldm<N, double>(a.sol, 0, s, S);
-    mac<0>(up, 1.0, et_, ppM);
+  const double bcb = bcf<double>(g, c, et(b));
+  const double bcmb = bcf<double>(g, c, -et(b));
+  Site cm = c;   // bc[M] at site x - b
+  cm.t = wrap(c.t - et(b), g.nt);
+  const double bcM_mb = bcf<double>(g, cm, et(M));
+  const double2* pbM = a.pd + (size_t)(b * 5 + M) * S;
+  const double2* pMb = a.pd + (size_t)(M * 5 + b) * S;
+  const Cx<double> bM = ldc<double>(pbM + s), Mb = ldc<double>(pMb + s);
+  const Cx<double> Mb_m = ldc<double>(pMb + mb), bM_m = ldc<double>(pbM + mb);
+  u = Cx<double>(0, 0);
+#pragma unroll
+  for (int q = 0; q < 2; q++) {
+    const double localG = (q == 0 ? -0.5 : 0.5) * a.G;
+    const double2* te = a.tr + (size_t)(q == 0 ? 11 : 10) * S;
+    const double2* TM = a.tr + (size_t)(5 * q + M) * S;
+    const double2* Tb = a.tr + (size_t)(5 * q + b) * S;
+    const Cx<double> te0 = ldc<double>(te + s), te_mb = ldc<double>(te + mb);
+    const Cx<double> TM0 = ldc<double>(TM + s);
+    const Cx<double> DbM = te0 * bM, DMb = te0 * Mb;
+    const Cx<double> DMb_mb = te_mb * Mb_m, DbM_mb = te_mb * bM_m;
+    Cx<double> plaq = DbM * (TM0 + bcM * ldc<double>(Tb + pM));
+    plaq = plaq + DMb_mb * (ldc<double>(Tb + mb) + bcmb * TM0);
+    Cx<double> adjt = DMb * (ldc<double>(Tb + s) + bcb * ldc<double>(TM + pb));
+    adjt = adjt + DbM_mb * (ldc<double>(TM + mb) + bcM_mb * ldc<double>(Tb + mbpM));
+    u = u + localG * plaq + conj(localG * adjt);
+    inv[q] = (-localG) * (DbM + bcmb * DMb_mb);
+  }
+}
+
+template <int N, int PAT>
+SUSY_D void ff_pattern(Mat<N, double>& acc, const FfArgs& a, int s, unsigned bcm, int M) {
+  constexpr bool SL = PAT == FF_SP || PAT == FF_DP;     // left factor from sol
+  constexpr bool AL = PAT == FF_PS || PAT == FF_DP;     // left factor adjointed
+  const int S = a.g.S;
+  const double pbc = (double)a.g.pbc;
+#pragma unroll 1
+  for (int t = 0; t < FF_ROWS; t++) {
+    const FfTerm T = c_ff[M][PAT][t];
+    const int il = a.nbrtab[(size_t)T.dl * S + s], ir = a.nbrtab[(size_t)T.dr * S + s];
+    const Mat<N, double> L = ldm<N, double, AL>(SL ? a.sol : a.psol, T.kl, il, S);
+    const Mat<N, double> R = ldm<N, double, !AL>(SL ? a.psol : a.sol, T.kr, ir, S);
+    mac<0>(acc, T.coef * bc_of<double>(bcm, T.b1, pbc) * bc_of<double>(bcm, T.b2, pbc), L, R);
+  }
+}
+
+// Fermion force of one pole: force[M] += amp f_U[M]^dag (update_h.c:943-958).
+//
+// A block is 32 sites of one link direction, its four warps the four operand
+// patterns (8 products each) and one of detF's four directions b each; the
+// warps' sums meet in shared memory and warp 0 adds U_M^-1 W U_M^-1 and
+// accumulates.  Gathers bound it, as they bound the operator (the same 320
+// operand matrices a site through L2).  The rows of the table are a rolled
+// loop so that a thread holds two operands and an accumulator: the kernel
+// this replaces unrolled all 44 products and 80 traces per link and lived in
+// local memory (per thread 8 KB of stack for NCOL 3, 45 KB for NCOL 4).
+// 12^3x24 U(3): 199 us a pole and 19 us of traces, against 1359 us.
+template <int N>
+constexpr int ff_blocks() { return N == 2 ? 6 : (N == 3 ? 4 : 2); }
+
+template <int N>
+__global__ void __launch_bounds__(FT, ff_blocks<N>()) k_fermion_force(FfArgs a) {
+  __shared__ double2 sacc[3][N * N][32];
+  __shared__ double2 sdet[4][3][32];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int M = blockIdx.x % NUMLINK;
+  const int s = (blockIdx.x / NUMLINK) * 32 + lane;
+  const int S = a.g.S;
+  const bool in = s < a.g.V;
+  Mat<N, double> acc;
+  acc.zero();
+  if (in) {
+    const Site c = site_of(a.g, s);
+    if (a.doG) {
+      Cx<double> u, inv[2];
+      ff_det(a, c, M, warp + (warp >= M), u, inv);
+      stc<double>(&sdet[warp][0][lane], u);
+      stc<double>(&sdet[warp][1][lane], inv[0]);
+      stc<double>(&sdet[warp][2][lane], inv[1]);
+    }
+    const unsigned bcm = bc_mask(a.g, c);
+    switch (warp) {
+      case 0: ff_pattern<N, FF_SP>(acc, a, s, bcm, M); break;
+      case 1: ff_pattern<N, FF_PS>(acc, a, s, bcm, M); break;
+      case 2: ff_pattern<N, FF_PD>(acc, a, s, bcm, M); break;
+      default: ff_pattern<N, FF_DP>(acc, a, s, bcm, M); break;
+    }
+    if (warp > 0) {
+#pragma unroll
+      for (int k = 0; k < N * N; k++)
+        sacc[warp - 1][k][lane] = make_double2(acc.e[k / N][k % N].re, acc.e[k / N][k % N].im);
+    }
+  }
+  __syncthreads();
+  if (warp > 0 || !in) return;
+#pragma unroll
+  for (int w = 0; w < 3; w++)
+#pragma unroll
+    for (int k = 0; k < N * N; k++) {
+      const double2 v = sacc[w][k][lane];
+      acc.e[k / N][k % N] = acc.e[k / N][k % N] + Cx<double>(v.x, v.y);
+    }
+  if (a.doG) {
+    Cx<double> d[3];
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      d[q] = Cx<double>(0, 0);
+#pragma unroll
+      for (int w = 0; w < 4; w++) {
+        const double2 v = sdet[w][q][lane];
+        d[q] = d[q] + Cx<double>(v.x, v.y);
+      }
+    }
+    // f += u U_M^-1 + U_M^-1 (inv_0 psi_M + inv_1 psi'_M^dag) U_M^-1, a row
+    // of the first product at a time; acc holds f^dag
+    const double2* ps = a.sol + (size_t)((1 + M) * N * N) * S + s;
+    const double2* pp = a.psol + (size_t)((1 + M) * N * N) * S + s;
+    Mat<N, double> ui = ldm<N, double>(a.Uinv, M, s, S);
+    Mat<N, double> w;
 #pragma unroll
     for (int i = 0; i < N; i++)
 #pragma unroll
-      for (int j = 0; j < N; j++) f.e[i][j] = Cx<double>(0.5 * up.e[j][i].re, -0.5 * up.e[j][i].im);
-  }
-  // V/P terms
+      for (int j = 0; j < N; j++)
+        w.e[i][j] = d[1] * ldc<double>(ps + (size_t)(i * N + j) * S) +
+                    d[2] * conj(ldc<double>(pp + (size_t)(j * N + i) * S));
 #pragma unroll
-  for (int nu = 0; nu < NUMLINK; nu++) {
-    if (nu == M) continue;
-    const double sg = M < nu ? 1.0 : -1.0;
-    const int q = 6 + pidx(M, nu);
-    const int mn = nbr(g, c, -ex(nu), -ey(nu), -ez(nu), -et(nu));
-    // -bc[M] psi_nu(x+M) chi'_{M nu}(x) + chi'_{M nu}(x-nu) psi_nu(x-nu)
-    Mat<N, double> P = ldm<N, double, true>(a.psol, q, s, S);
-    Mat<N, double> ps = ldm<N, double>(a.sol, 1 + nu, pM, S);
-    mac<0>(f, -bcM * sg, ps, P);
-    P = ldm<N, double, true>(a.psol, q, mn, S);
-    ps = ldm<N, double>(a.sol, 1 + nu, mn, S);
-    mac<0>(f, sg, P, ps);
-    // psi'_nu(x+M) bc[M] chi_{M nu}(x) - chi_{M nu}(x-nu) psi'_nu(x-nu)
-    Mat<N, double> C = ldm<N, double>(a.sol, q, s, S);
-    Mat<N, double> pp = ldm<N, double, true>(a.psol, 1 + nu, pM, S);
-    mac<0>(f, bcM * sg, pp, C);
-    C = ldm<N, double>(a.sol, q, mn, S);
-    pp = ldm<N, double, true>(a.psol, 1 + nu, mn, S);
-    mac<0>(f, -sg, C, pp);
-  }
-  if (a.doG) {
-    detF_term<N, M, true>(f, a, c);
-    detF_term<N, M, false>(f, a, c);
-  }
-  typedef Compl4<M> K;
-  fq_terms<N, M, K::K0, K::K1, K::K2, K::K3>(f, a, c);
-  fq_terms<N, M, K::K2, K::K3, K::K0, K::K1>(f, a, c);
-  fq_terms<N, M, K::K0, K::K2, K::K1, K::K3>(f, a, c);
-  fq_terms<N, M, K::K1, K::K3, K::K0, K::K2>(f, a, c);
-  fq_terms<N, M, K::K0, K::K3, K::K1, K::K2>(f, a, c);
-  fq_terms<N, M, K::K1, K::K2, K::K0, K::K3>(f, a, c);
-  return f;
-}
-
-template <int N>
-__global__ void __launch_bounds__(FT) k_fermion_force(FfArgs a) {
-  const int M = blockIdx.x % NUMLINK;
-  const int s = (blockIdx.x / NUMLINK) * FT + threadIdx.x;
-  if (s >= a.g.V) return;
-  const Site c = site_of(a.g, s);
-  Mat<N, double> f;
-  switch (M) {
-    case 0: f = fforce_out<N, 0>(a, c); break;
-    case 1: f = fforce_out<N, 1>(a, c); break;
-    case 2: f = fforce_out<N, 2>(a, c); break;
-    case 3: f = fforce_out<N, 3>(a, c); break;
-    default: f = fforce_out<N, 4>(a, c); break;
-  }
-  // fullforce[M] += amp f_U^dag  (update_h.c:943-958)
-  Mat<N, double> acc = ldm<N, double>(a.force, M, s, a.g.S);
+    for (int i = 0; i < N; i++) {
+      Cx<double> row[N];
 #pragma unroll
-  for (int i = 0; i < N; i++)
+      for (int j = 0; j < N; j++) {
+        row[j] = Cx<double>(0, 0);
 #pragma unroll
-    for (int j = 0; j < N; j++) {
-      acc.e[i][j].re += a.amp * f.e[j][i].re;
-      acc.e[i][j].im -= a.amp * f.e[j][i].im;
+        for (int k = 0; k < N; k++) row[j] = row[j] + ui.e[i][k] * w.e[k][j];
+        if (i == j) row[j] = row[j] + d[0];
+      }
+#pragma unroll
+      for (int j = 0; j < N; j++) {
+        Cx<double> f(0, 0);
+#pragma unroll
+        for (int k = 0; k < N; k++) f = f + row[k] * ui.e[k][j];
+        acc.e[j][i] = acc.e[j][i] + conj(f);
+      }
     }
-  stm<N, double>(a.force, M, s, a.g.S, acc);
+  }
+  double2* pf = a.force + (size_t)(M * N * N) * S + s;
+#pragma unroll
+  for (int k = 0; k < N * N; k++) {
+    double2 v = pf[(size_t)k * S];
+    v.x += a.amp * acc.e[k / N][k % N].re;
+    v.y += a.amp * acc.e[k / N][k % N].im;
+    pf[(size_t)k * S] = v;
+  }
 }
 
 // mom -= eps force; partials of |force|^2   (update_h.c:965-971)
@@ -452,25 +515,32 @@ static inline int nbk(long n, int t) { return (int)((n + t - 1) / t); }
 int force_blocks(const Geo& g) { return nbk(g.V, FT) * NUMLINK; }
 int site_blocks(const Geo& g) { return nbk(g.V, FT); }
 
-void fermion_force_pole(const Geo& g, int N, const void* U, const void* Uinv, const void* pd,
-                        const void* sol, const void* psol, void* force, double amp, double G,
-                        cudaStream_t st) {
+template <int N>
+static void launch_fermion_force(const FfArgs& a, double2* tr, cudaStream_t st) {
+  if (a.doG)
+    count_launch(), k_ff_traces<N><<<dim3(nbk(a.g.V, FT), NUMLINK + 1), FT, 0, st>>>(a, tr);
+  count_launch(), k_fermion_force<N><<<nbk(a.g.V, 32) * NUMLINK, FT, 0, st>>>(a);
+}
+
+void fermion_force_pole(const Geo& g, int N, const void* Uinv, const void* pd,
+                        const void* sol, const void* psol, void* force, void* tr,
+                        const int* nbrtab, double amp, double G, cudaStream_t st) {
   FfArgs a;
   a.g = g;
-  a.U = (const double2*)U;
   a.Uinv = (const double2*)Uinv;
   a.pd = (const double2*)pd;
   a.sol = (const double2*)sol;
   a.psol = (const double2*)psol;
   a.force = (double2*)force;
+  a.tr = (const double2*)tr;
+  a.nbrtab = nbrtab;
   a.amp = amp;
   a.G = G;
   a.doG = G > 1e-8;
-  const int nb = force_blocks(g);
   switch (N) {
-    case 2: count_launch(), k_fermion_force<2><<<nb, FT, 0, st>>>(a); break;
-    case 3: count_launch(), k_fermion_force<3><<<nb, FT, 0, st>>>(a); break;
-    case 4: count_launch(), k_fermion_force<4><<<nb, FT, 0, st>>>(a); break;
+    case 2: launch_fermion_force<2>(a, (double2*)tr, st); break;
+    case 3: launch_fermion_force<3>(a, (double2*)tr, st); break;
+    case 4: launch_fermion_force<4>(a, (double2*)tr, st); break;
   }
 }
 

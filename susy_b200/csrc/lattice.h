@@ -30,6 +30,7 @@ struct susy_b200_lattice {
   int* nbrtab = nullptr;  // neighbour index table of the table-driven operator
   void* trace[2] = {};    // determinant traces of FOP_SITE_MAJOR_TR (FP64, FP32);
                           // each solver context owns its own
+  void* ftrace = nullptr; // traces the fermion force's determinant terms read
   susy::MsState* ms = nullptr;
   void* tf64[SUSY_NSCRATCH] = {};
   void* tf32[SUSY_NSCRATCH] = {};
