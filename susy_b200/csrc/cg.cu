@@ -68,98 +68,121 @@ __global__ void k_ms_init(MsState* st, const double* partials, int np, int maxcg
   }
 }
 
-SUSY_D double block_reduce_all(double v, double* sh) {
-  sh[threadIdx.x] = v;
+// Sum of np partials over the block of ST threads, on every thread
+// (sh: ST / 32 words)
+template <bool L2>
+SUSY_D double sum_partials(const double* partials, int np, double* sh) {
+  double v = 0.0;
+#pragma unroll 4
+  for (int i = threadIdx.x; i < np; i += ST) v += L2 ? __ldcg(partials + i) : partials[i];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
   __syncthreads();
-  for (int o = ST / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-    __syncthreads();
-  }
-  return sh[0];
+  double r = 0.0;
+#pragma unroll
+  for (int i = 0; i < ST / 32; i++) r += sh[i];
+  return r;
 }
 
-// The scalar recurrences after the operator, run by one block of ST threads
+// The scalar recurrences after the operator, run by one block of ST threads.
+// Thread j holds shift j: its divisions (two per shift) are a serial chain of
+// a few hundred cycles, which one thread looping over 15 shifts made 5.4 us
+// of this step and 10 us of the next at any lattice size.
 SUSY_D void scalars1_block(MsState* st, const double* partials, int np, double* sh) {
   if (st->skip) {
     if (threadIdx.x == 0) st->skip_b = 1;
     return;
   }
-  double v = 0.0;
-  for (int i = threadIdx.x; i < np; i += ST) v += partials[i];
-  const double cd = block_reduce_all(v, sh);
-  if (threadIdx.x != 0) return;
-  st->skip_b = 0;
-  st->cd = cd;
-  st->iter += 1;
-  const double b0 = -st->rsq / cd;
-  st->beta_i[0] = b0;
-  st->zeta_ip1[0] = 1.0;
-  const double s0 = st->shift[0];
-  for (int j = 1; j < st->nshift; j++) {
-    if (st->converged[j]) continue;
-    double z = st->zeta_i[j] * st->zeta_im1[j] * st->beta_im1[0];
-    const double c1 = b0 * st->alpha[0] * (st->zeta_im1[j] - st->zeta_i[j]);
-    const double c2 = st->zeta_im1[j] * st->beta_im1[0] * (1.0 - (st->shift[j] - s0) * b0);
+  const int j = threadIdx.x;
+  const bool mine = j < st->nshift && j > 0 && !st->converged[j];
+  const double rsq = st->rsq, a0 = st->alpha[0], bm0 = st->beta_im1[0];
+  double zi = 1.0, zm = 1.0, ds = 0.0;
+  if (mine) {
+    zi = st->zeta_i[j];
+    zm = st->zeta_im1[j];
+    ds = st->shift[j] - st->shift[0];
+  }
+  const double cd = sum_partials<false>(partials, np, sh);
+  const double b0 = -rsq / cd;
+  if (j == 0) {
+    st->skip_b = 0;
+    st->cd = cd;
+    st->iter += 1;
+    st->beta_i[0] = b0;
+    st->zeta_ip1[0] = 1.0;
+  }
+  if (mine) {
+    double z = zi * zm * bm0;
+    const double c1 = b0 * a0 * (zm - zi);
+    const double c2 = zm * bm0 * (1.0 - ds * b0);
     z /= c1 + c2;
     st->zeta_ip1[j] = z;
-    st->beta_i[j] = b0 * z / st->zeta_i[j];
+    st->beta_i[j] = b0 * z / zi;
   }
 }
 
 __global__ void k_ms_scalars1(MsState* st, const double* partials, int np) {
-  __shared__ double sh[ST];
+  __shared__ double sh[ST / 32];
   scalars1_block(st, partials, np, sh);
 }
 
 // The scalar recurrences after the residual update, run by one block of ST
-// threads: its own kernel, or the last block of the fused residual update
-// (partials read from L2: other blocks wrote them)
+// threads (thread j: shift j): its own kernel, or the last block of the
+// fused residual update (partials read from L2: other blocks wrote them)
 SUSY_D void scalars2_block(MsState* st, const double* partials, int np, double* sh) {
-  double v = 0.0;
-  for (int i = threadIdx.x; i < np; i += ST) v += __ldcg(partials + i);
-  const double rsqnew = block_reduce_all(v, sh);
-  if (threadIdx.x != 0) return;
-  const double a0 = rsqnew / st->rsq;
-  st->alpha[0] = a0;
-  st->active_p[0] = 1;
-  for (int j = 1; j < st->nshift; j++) {
-    st->active_p[j] = !st->converged[j];
-    if (st->converged[j]) continue;
-    st->alpha[j] = a0 * st->zeta_ip1[j] * st->beta_i[j] / (st->zeta_i[j] * st->beta_i[0]);
+  const int j = threadIdx.x;
+  const bool mine = j < st->nshift;
+  const double rsq = st->rsq;
+  const int t = st->record && st->blk_len < MS_BLK ? st->blk_len : -1;
+  double bi = 0.0, zi = 1.0, zp = 1.0, al = 0.0, b0 = 1.0;
+  bool live = false;
+  if (mine) {
+    live = j == 0 || !st->converged[j];
+    bi = st->beta_i[j];
+    b0 = st->beta_i[0];
+    zi = st->zeta_i[j];
+    zp = st->zeta_ip1[j];
+    al = st->alpha[j];
   }
-  if (st->record && st->blk_len < MS_BLK) {
-    // this iteration's coefficients, before this iteration's freeze test:
-    // a shift frozen in an earlier iteration took no step in this one
-    const int t = st->blk_len++;
-    for (int j = 0; j < st->nshift; j++) {
-      const bool live = j == 0 || !st->converged[j];
-      st->hb[t][j] = live ? st->beta_i[j] : 0.0;
-      st->hz[t][j] = j == 0 ? 1.0 : st->zeta_ip1[j];
-      st->ha[t][j] = st->alpha[j];
+  // every thread has read the state above once the sum's barrier is passed
+  const double rsqnew = sum_partials<true>(partials, np, sh);
+  const double a0 = rsqnew / rsq;
+  if (mine) {
+    if (j == 0)
+      al = a0;
+    else if (live)
+      al = a0 * zp * bi / (zi * b0);
+    st->alpha[j] = al;
+    st->active_p[j] = live;
+    if (t >= 0) {
+      // this iteration's coefficients, before this iteration's freeze test:
+      // a shift frozen in an earlier iteration took no step in this one
+      st->hb[t][j] = live ? bi : 0.0;
+      st->hz[t][j] = j == 0 ? 1.0 : zp;
+      st->ha[t][j] = al;
+    }
+    st->pz[j] = zp;
+    st->pa[j] = al;
+    st->pact[j] = live;
+    // converged[j] = the iteration at which shift j froze (>= 1; 0 = live)
+    if (j > 0 && live && rsqnew * zp * zp <= st->rsqfreeze) {
+      st->converged[j] = st->iter;
+    } else if (live) {
+      st->beta_im1[j] = bi;
+      st->zeta_im1[j] = zi;
+      st->zeta_i[j] = zp;
     }
   }
-  for (int j = 0; j < st->nshift; j++) {
-    st->pz[j] = st->zeta_ip1[j];
-    st->pa[j] = st->alpha[j];
-    st->pact[j] = st->active_p[j];
+  if (j == 0) {
+    if (t >= 0) st->blk_len = t + 1;
+    st->rsq = rsqnew;
+    st->skip = (rsqnew <= st->rsqstop || st->iter >= st->maxcg) ? 1 : 0;
   }
-  st->rsq = rsqnew;
-  for (int j = 1; j < st->nshift; j++) {
-    if (st->converged[j]) continue;
-    // converged[j] = the iteration at which shift j froze (>= 1; 0 = live)
-    if (rsqnew * st->zeta_ip1[j] * st->zeta_ip1[j] <= st->rsqfreeze) st->converged[j] = st->iter;
-  }
-  for (int j = 0; j < st->nshift; j++) {
-    if (st->converged[j]) continue;
-    st->beta_im1[j] = st->beta_i[j];
-    st->zeta_im1[j] = st->zeta_i[j];
-    st->zeta_i[j] = st->zeta_ip1[j];
-  }
-  st->skip = (rsqnew <= st->rsqstop || st->iter >= st->maxcg) ? 1 : 0;
 }
 
 __global__ void k_ms_scalars2(MsState* st, const double* partials, int np) {
-  __shared__ double sh[ST];
+  __shared__ double sh[ST / 32];
   if (st->skip) return;
   scalars2_block(st, partials, np, sh);
 }
@@ -472,7 +495,8 @@ template <typename MT, typename RT>
 __global__ void __launch_bounds__(UT) k_msb_update_r(MsState* st, MsBlockVecs v, long n,
                                                      double* part) {
   static_assert(UT == ST, "the last block runs the ST-thread scalar step");
-  __shared__ double sh[ST];
+  static_assert(MS_MAXS <= ST, "one thread per shift");
+  __shared__ double sh[ST / 32];
   __shared__ int last;
   if (st->skip) return;
   const int it = st->iter;
@@ -752,13 +776,13 @@ SUSY_D int vblock_lattice(const MsLat* L, int nl, int b) {
 }
 
 __global__ void k_msbat_scalars1(const MsLat* L) {
-  __shared__ double sh[ST];
+  __shared__ double sh[ST / 32];
   const MsLat& l = L[blockIdx.x];
   scalars1_block(l.st, l.part0, l.np0, sh);
 }
 
 __global__ void k_msbat_scalars2(const MsLat* L) {
-  __shared__ double sh[ST];
+  __shared__ double sh[ST / 32];
   const MsLat& l = L[blockIdx.x];
   if (l.st->skip) return;
   scalars2_block(l.st, l.part1, l.vblocks, sh);

@@ -232,3 +232,28 @@ def test_host_congrad_multi_early_copies(solver):
         lat.congrad_multi(src, outs, shifts, 20000, 1e-20)
     for a, b in zip(pinned, pageable):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("blocked", [0, 1])
+@pytest.mark.parametrize("norder", [1, 2, 32])
+def test_shift_counts_at_the_edges(norder, blocked):
+    """One thread per shift runs the scalar recurrences: a single shift, two,
+    and the most the state holds, with shifts that freeze in the first
+    iterations, against the oracle (tolerances as above)."""
+    dims, N = (4, 2, 4, 4), 2
+    U = synth.links(dims, N, 0.2, 4)
+    lat = Lattice(dims, N, pbc=-1, G=0.05)
+    lat.set_links(synth.to_ref(dims, U))
+    lat.cg_blocked(blocked)
+    geo = O.Geometry(dims, -1)
+    prm = O.Params(G=0.05, N=N)
+    der = O.compute_derived(geo, prm, U)
+    src = synth.tf_source(dims, N, seed=8)
+    shifts = synth.geometric_shifts(norder, 1e-3, 1e6) if norder > 1 else np.array([0.01])
+    want, wit, _ = O.congrad_multi(geo, prm, U, der, src, shifts, 5000, 1e-18)
+    psim = [np.zeros(lat.tf_doubles) for _ in shifts]
+    it, _ = lat.congrad_multi(synth.to_ref(dims, src), psim, shifts, 5000, 1e-18)
+    assert abs(it - wit) <= 1
+    for j in range(norder):
+        got = synth.from_ref(dims, psim[j], 16, N)
+        assert np.abs(got - want[j]).max() / np.abs(want[j]).max() < 1e-8
