@@ -236,8 +236,8 @@ susy_b200_lattice* solver_shadow(susy_b200_lattice* h) {
     }
     c->stream = c->own_stream;
     c->ms = (MsState*)dalloc(c, sizeof(MsState));
-    c->trace[0] = dalloc(c, 5 * c->g.S * sizeof(double2));
-    c->trace[1] = dalloc(c, 5 * c->g.S * sizeof(float2));
+    c->trace[0] = dalloc(c, 6 * c->g.S * sizeof(double2));
+    c->trace[1] = dalloc(c, 6 * c->g.S * sizeof(float2));
     if (!c->ms || !c->trace[0] || !c->trace[1]) {
       susy_b200_destroy(c);
       return nullptr;
@@ -315,8 +315,8 @@ susy_b200_lattice* susy_b200_create(const susy_b200_params* p) {
   h->stage = dalloc(h, (size_t)h->g.V * NTF * mat_c(h) * 2 * sizeof(double));
   h->ms = (MsState*)dalloc(h, sizeof(MsState));
   h->nbrtab = (int*)dalloc(h, (size_t)fop_ndisp() * h->g.S * sizeof(int));
-  h->trace[0] = dalloc(h, 5 * h->g.S * sizeof(double2));
-  h->trace[1] = dalloc(h, 5 * h->g.S * sizeof(float2));
+  h->trace[0] = dalloc(h, 6 * h->g.S * sizeof(double2));
+  h->trace[1] = dalloc(h, 6 * h->g.S * sizeof(float2));
   if (h->nbrtab) build_nbr_table(h->g, h->nbrtab, h->stream);
   if (h->err) {
     susy_b200_destroy(h);

@@ -279,6 +279,9 @@ int fermion_op(const Geo& g, int N, const void* U, const void* Uinv, const void*
   a.trace = (T*)trace;
   if (variant == FOP_SITE_MAJOR_TR && !trace) variant = FOP_SITE_MAJOR_FRONT;
   if (variant == FOP_ROWS) return fermion_op_rows<R>(a, N, sign, st);
+  const bool rolling = variant == FOP_ROLLING || variant == FOP_ROLLING_WIDE;
+  if (rolling && !trace) variant = FOP_SITE_MAJOR_FRONT;
+  else if (rolling) return fermion_op_rolling<R>(a, N, sign, variant == FOP_ROLLING_WIDE, st);
   if (variant >= FOP_COMPACT) return fermion_op_compact<R>(a, N, sign, variant, st);
   a.comp_major = variant == FOP_MAT_CM;
   switch (N) {

@@ -28,12 +28,6 @@ namespace susy {
 __constant__ FTerm c_terms[MAX_TERMS];
 __constant__ short c_pat_start[NTF][NPAT + 1];
 __constant__ char4 c_disp[MAX_DISP];
-// Distinct displacements of each output component's products (at most 10):
-// the blocks of the shared-index kernels preload those neighbour indices
-// into shared memory; FTerm.sl / .sr are a product's slots in that list.
-constexpr int MAX_SLOTS = 12;
-__constant__ int8_t c_slot_disp[NTF][MAX_SLOTS];
-__constant__ int8_t c_nslot[NTF];
 
 const TermBuilder& fop_terms() {
   static const TermBuilder tb = [] {
@@ -57,34 +51,17 @@ int upload_fop_terms(int device, cudaStream_t st) {
   const TermBuilder& tb = fop_terms();
   std::vector<FTerm> flat;
   short start[NTF][NPAT + 1];
-  int8_t slot_disp[NTF][MAX_SLOTS] = {};
-  int8_t nslot[NTF] = {};
-  auto slot = [&](int c, int d) -> int {
-    for (int j = 0; j < nslot[c]; j++)
-      if (slot_disp[c][j] == d) return j;
-    if (nslot[c] >= MAX_SLOTS) return -1;
-    slot_disp[c][nslot[c]] = (int8_t)d;
-    return nslot[c]++;
-  };
   for (int c = 0; c < NTF; c++)
     for (int p = 0; p < NPAT; p++) {
       start[c][p] = (short)flat.size();
-      for (FTerm T : tb.terms[c][p]) {
-        const int a = slot(c, T.dl), b = slot(c, T.dr);
-        if (a < 0 || b < 0) return -1;
-        T.sl = (int8_t)a;
-        T.sr = (int8_t)b;
-        flat.push_back(T);
-      }
+      for (const FTerm& T : tb.terms[c][p]) flat.push_back(T);
       start[c][p + 1] = (short)flat.size();
     }
   if ((int)flat.size() > MAX_TERMS || (int)tb.disp.size() > MAX_DISP) return -1;
   cudaMemcpyToSymbol(c_terms, flat.data(), flat.size() * sizeof(FTerm));
   cudaMemcpyToSymbol(c_pat_start, start, sizeof(start));
   cudaMemcpyToSymbol(c_disp, tb.disp.data(), tb.disp.size() * sizeof(char4));
-  cudaMemcpyToSymbol(c_slot_disp, slot_disp, sizeof(slot_disp));
-  cudaMemcpyToSymbol(c_nslot, nslot, sizeof(nslot));
-  if (upload_force_terms() != 0) return -2;
+  if (upload_force_terms() != 0 || upload_rolling_terms() != 0) return -2;
   if (cudaGetLastError() != cudaSuccess) return -2;
   prefer_l1_grouped<double>();
   prefer_l1_grouped<float>();
@@ -221,11 +198,8 @@ fermion_op_compact_kernel(FopArgs<R> a) {
 // depends on the precision (the autotuner decides).
 
 // PP = false: one operand buffer, no prefetch (fewest registers).
-// shn != nullptr: neighbour indices from the block's shared-memory copy
-// (shn[slot * CT_THREADS + threadIdx.x]) instead of the global table.
 template <int N, typename R, int SIGN, int PAT, bool PP, typename ACC>
-SUSY_D void run_pattern_pp(ACC& acc, const FopArgs<R>& a, int s, unsigned bcm, int t0, int t1,
-                           const int* shn = nullptr) {
+SUSY_D void run_pattern_pp(ACC& acc, const FopArgs<R>& a, int s, unsigned bcm, int t0, int t1) {
   constexpr bool LF = (PAT == P_FU || PAT == P_FUD);
   constexpr bool RF = !LF;
   constexpr bool AL = (PAT == P_UDF) ^ (LF && SIGN < 0);
@@ -239,8 +213,8 @@ SUSY_D void run_pattern_pp(ACC& acc, const FopArgs<R>& a, int s, unsigned bcm, i
 #pragma unroll 1
     for (int t = t0; t < t1; t++) {
       const FTerm T = c_terms[t];
-      const int il = shn ? shn[T.sl * CT_THREADS + threadIdx.x] : a.nbrtab[(size_t)T.dl * S + s];
-      const int ir = shn ? shn[T.sr * CT_THREADS + threadIdx.x] : a.nbrtab[(size_t)T.dr * S + s];
+      const int il = a.nbrtab[(size_t)T.dl * S + s];
+      const int ir = a.nbrtab[(size_t)T.dr * S + s];
       const Mat<N, R> L = ldm<N, R, AL>(fl, T.kl, il, S);
       const Mat<N, R> Rm = ldm<N, R, AR>(fr, T.kr, ir, S);
       acc.add((R)T.coef * bc_of<R>(bcm, T.bcdt, pbc) * ((LF ? T.kl : T.kr) ? (R)1 : a.eta_scale), L, Rm);
@@ -301,13 +275,10 @@ SUSY_D int front_block(int b, int ntile, int& k) {
 
 // Block order: site-major (SM = true) or component-major; PP: two operand
 // buffers (prefetch) or one.
-// SHN: the block first copies its output component's neighbour indices
-// (at most MAX_SLOTS displacements x CT_THREADS sites) into shared memory,
-// so a product's operand loads no longer wait on a global index load.
 // FRONT (with SM): the site component's blocks first, then the others
 // site-major (front_block).  TR: detLtoS from the pre-pass's traces.
-template <int N, typename R, int SIGN, bool SM, bool PP, int MINB, bool SHN = false,
-          bool FRONT = false, bool TR = false>
+template <int N, typename R, int SIGN, bool SM, bool PP, int MINB, bool FRONT = false,
+          bool TR = false>
 __global__ void __launch_bounds__(CT_THREADS, MINB)
 fermion_op_pp_kernel(FopArgs<R> a) {
   if (a.skip && *a.skip) return;
@@ -319,25 +290,16 @@ fermion_op_pp_kernel(FopArgs<R> a) {
     tile = SM ? blockIdx.x / NTF : blockIdx.x % a.nsb;
   }
   const int s = tile * CT_THREADS + threadIdx.x;
-  __shared__ int shn[SHN ? MAX_SLOTS * CT_THREADS : 1];
-  if (SHN) {
-    const int ns = c_nslot[comp];
-    for (int j = 0; j < ns; j++)
-      shn[j * CT_THREADS + threadIdx.x] =
-          s < a.g.V ? a.nbrtab[(size_t)c_slot_disp[comp][j] * a.g.S + s] : 0;
-    __syncthreads();
-  }
-  const int* sh = SHN ? shn : nullptr;
   double part = 0.0;
   if (s < a.g.V) {
     const Site c = site_of(a.g, s);
     const unsigned bcm = bc_mask(a.g, c);
     AccMat<N, R> acc;
     acc.zero();
-    run_pattern_pp<N, R, SIGN, P_UF, PP>(acc, a, s, bcm, c_pat_start[comp][0], c_pat_start[comp][1], sh);
-    run_pattern_pp<N, R, SIGN, P_FU, PP>(acc, a, s, bcm, c_pat_start[comp][1], c_pat_start[comp][2], sh);
-    run_pattern_pp<N, R, SIGN, P_FUD, PP>(acc, a, s, bcm, c_pat_start[comp][2], c_pat_start[comp][3], sh);
-    run_pattern_pp<N, R, SIGN, P_UDF, PP>(acc, a, s, bcm, c_pat_start[comp][3], c_pat_start[comp][4], sh);
+    run_pattern_pp<N, R, SIGN, P_UF, PP>(acc, a, s, bcm, c_pat_start[comp][0], c_pat_start[comp][1]);
+    run_pattern_pp<N, R, SIGN, P_FU, PP>(acc, a, s, bcm, c_pat_start[comp][1], c_pat_start[comp][2]);
+    run_pattern_pp<N, R, SIGN, P_FUD, PP>(acc, a, s, bcm, c_pat_start[comp][2], c_pat_start[comp][3]);
+    run_pattern_pp<N, R, SIGN, P_UDF, PP>(acc, a, s, bcm, c_pat_start[comp][3], c_pat_start[comp][4]);
     Mat<N, R> out = acc.get();
     part = fop_finish<N, R, SIGN, TR>(out, a, c, comp);
   }
@@ -451,8 +413,7 @@ static int launch_compact(FopArgs<R> a, int sign, cudaStream_t st) {
   return nblk;
 }
 
-template <int N, typename R, bool SM, bool PP, int MINB = 1, bool SHN = false, bool FRONT = false,
-          bool TR = false>
+template <int N, typename R, bool SM, bool PP, int MINB = 1, bool FRONT = false, bool TR = false>
 static int launch_pp(FopArgs<R> a, int sign, cudaStream_t st) {
   a.nsb = (a.g.V + CT_THREADS - 1) / CT_THREADS;
   const int nblk = a.nsb * NTF;
@@ -464,9 +425,9 @@ static int launch_pp(FopArgs<R> a, int sign, cudaStream_t st) {
       count_launch(), k_det_traces<N, R, true><<<nb, CT_THREADS, 0, st>>>(a);
   }
   if (sign > 0)
-    count_launch(), fermion_op_pp_kernel<N, R, 1, SM, PP, MINB, SHN, FRONT, TR><<<nblk, CT_THREADS, 0, st>>>(a);
+    count_launch(), fermion_op_pp_kernel<N, R, 1, SM, PP, MINB, FRONT, TR><<<nblk, CT_THREADS, 0, st>>>(a);
   else
-    count_launch(), fermion_op_pp_kernel<N, R, -1, SM, PP, MINB, SHN, FRONT, TR><<<nblk, CT_THREADS, 0, st>>>(a);
+    count_launch(), fermion_op_pp_kernel<N, R, -1, SM, PP, MINB, FRONT, TR><<<nblk, CT_THREADS, 0, st>>>(a);
   return nblk;
 }
 
@@ -625,32 +586,20 @@ int fermion_op_compact(const FopArgs<R>& a, int N, int sign, int variant, cudaSt
         case 3: return launch_pp<3, R, true, false, 4>(a, sign, st);
         default: return launch_pp<4, R, true, false, 4>(a, sign, st);
       }
-    case FOP_SITE_MAJOR_SHN:
-      switch (N) {
-        case 2: return launch_pp<2, R, true, false, 4, true>(a, sign, st);
-        case 3: return launch_pp<3, R, true, false, 4, true>(a, sign, st);
-        default: return launch_pp<4, R, true, false, 4, true>(a, sign, st);
-      }
-    case FOP_COMP_MAJOR_SHN:
-      switch (N) {
-        case 2: return launch_pp<2, R, false, false, 8, true>(a, sign, st);
-        case 3: return launch_pp<3, R, false, false, 8, true>(a, sign, st);
-        default: return launch_pp<4, R, false, false, 8, true>(a, sign, st);
-      }
     case FOP_SITE_MAJOR_FRONT: {
       constexpr int MB = sizeof(R) == 8 ? 4 : 8;
       switch (N) {
-        case 2: return launch_pp<2, R, true, false, MB, false, true>(a, sign, st);
-        case 3: return launch_pp<3, R, true, false, MB, false, true>(a, sign, st);
-        default: return launch_pp<4, R, true, false, MB, false, true>(a, sign, st);
+        case 2: return launch_pp<2, R, true, false, MB, true>(a, sign, st);
+        case 3: return launch_pp<3, R, true, false, MB, true>(a, sign, st);
+        default: return launch_pp<4, R, true, false, MB, true>(a, sign, st);
       }
     }
     case FOP_SITE_MAJOR_TR: {
       constexpr int MB = sizeof(R) == 8 ? 4 : 8;
       switch (N) {
-        case 2: return launch_pp<2, R, true, false, MB, false, true, true>(a, sign, st);
-        case 3: return launch_pp<3, R, true, false, MB, false, true, true>(a, sign, st);
-        default: return launch_pp<4, R, true, false, MB, false, true, true>(a, sign, st);
+        case 2: return launch_pp<2, R, true, false, MB, true, true>(a, sign, st);
+        case 3: return launch_pp<3, R, true, false, MB, true, true>(a, sign, st);
+        default: return launch_pp<4, R, true, false, MB, true, true>(a, sign, st);
       }
     }
     case FOP_GROUPED:

@@ -1,0 +1,311 @@
+// The fermion operator with rolling operand loads (the products of
+// fop_table.cuh).
+//
+// Every output component has exactly two products with each link direction
+// C, one U_C F and one F U_C with the same source component F and the same
+// adjoint of U_C: chi'_AB takes U_A, U_B with psi_B, psi_A and Ubar_C with the
+// plaquette opposite to it, psi'_B takes U_e with chi_eB and Ubar_B with eta,
+// eta' takes Ubar_e with psi_e.  So one loop over C with a U F and an F U
+// product in it serves all sixteen components.
+#include <vector>
+#include "common.cuh"
+#include "fop.cuh"
+#include "fop_table.cuh"
+#include "kernels.h"
+
+namespace susy {
+
+constexpr int RL_THREADS = 128;
+
+// The two products of output component c with direction C:
+//   cuf op(U_C(disp uuf)) F_k(disp duf)  +  cfu F_k(disp dfu) op(U_C(disp ufu))
+struct RlTerm {
+  int8_t k, adj;
+  int8_t uuf, ufu;
+  int8_t duf, dfu;
+  int8_t buf, bfu;   // time displacements of the BC factors
+  float cuf, cfu;
+};
+__constant__ RlTerm c_rl[NUMLINK][NTF];
+
+int upload_rolling_terms() {
+  const TermBuilder& tb = fop_terms();
+  RlTerm t[NUMLINK][NTF] = {};
+  int nuf[NUMLINK][NTF] = {}, nfu[NUMLINK][NTF] = {};
+  for (int c = 0; c < NTF; c++)
+    for (int p = 0; p < NPAT; p++)
+      for (const FTerm& T : tb.terms[c][p]) {
+        const bool uf = p == P_UF || p == P_UDF;
+        const int C = uf ? T.kl : T.kr, k = uf ? T.kr : T.kl;
+        const int adj = p == P_FUD || p == P_UDF;
+        RlTerm& S = t[C][c];
+        if (nuf[C][c] + nfu[C][c] > 0 && (S.k != k || S.adj != adj)) return -1;
+        S.k = (int8_t)k;
+        S.adj = (int8_t)adj;
+        if (uf) {
+          S.uuf = T.dl;
+          S.duf = T.dr;
+          S.buf = T.bcdt;
+          S.cuf = T.coef;
+          nuf[C][c]++;
+        } else {
+          S.ufu = T.dr;
+          S.dfu = T.dl;
+          S.bfu = T.bcdt;
+          S.cfu = T.coef;
+          nfu[C][c]++;
+        }
+      }
+  for (int C = 0; C < NUMLINK; C++)
+    for (int c = 0; c < NTF; c++)
+      if (nuf[C][c] != 1 || nfu[C][c] != 1) return -1;
+  return cudaMemcpyToSymbol(c_rl, t, sizeof(t)) == cudaSuccess ? 0 : -2;
+}
+
+template <typename R>
+SUSY_D void cfma(Cx<R>& c, const Cx<R>& a, const Cx<R>& b) {
+  c.re = fma(a.re, b.re, c.re);
+  c.re = fma(-a.im, b.im, c.re);
+  c.im = fma(a.re, b.im, c.im);
+  c.im = fma(a.im, b.re, c.im);
+}
+
+// One product's link operand: element (i, j) of op(U) is p[i * si + j * sj],
+// its imaginary part times the sign of the adjoint
+template <typename R>
+struct LinkPtr {
+  const typename CT<R>::T* p;
+  int si, sj;
+};
+
+// Element (i, j) of F, or of its adjoint without the conjugation (that is
+// left to the use: a sign here would wait for the load)
+template <int N, typename R, bool ADJF>
+SUSY_D Cx<R> ld_src(const typename CT<R>::T* p, int i, int j, int S) {
+  return ldc<R>(p + (size_t)((ADJF ? j * N + i : i * N + j) * S));
+}
+template <typename R>
+SUSY_D Cx<R> ld_link(const LinkPtr<R>& u, int i, int j) {
+  return ldc<R>(u.p + i * u.si + j * u.sj);
+}
+
+// acc += op(U) F (UF) or F op(U), op(U)'s elements times (c, ci) as they are
+// used.  The sum runs over the inner index outermost: a column of the left
+// factor and a row of the right one are dead after each step, and the same
+// registers take the next product's operands (of the other kind) in the
+// order it will use them.  So the loads of the next product are in flight
+// while this one computes, at no cost in registers.
+template <int N, typename R, bool UF, bool ADJF, bool MORE = true>
+SUSY_D void mac_roll(Mat<N, R>& acc, R c, R ci, Mat<N, R>& U, Mat<N, R>& F,
+                     const LinkPtr<R>& nu, const typename CT<R>::T* nf, int S) {
+  Mat<N, R> U2, F2;
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    Cx<R> u[N], f[N];
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      const Cx<R> v = UF ? U.e[i][k] : U.e[k][i];
+      u[i] = Cx<R>(c * v.re, ci * v.im);
+      f[i] = UF ? F.e[k][i] : F.e[i][k];
+      if (ADJF) f[i] = conj(f[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      if (!MORE) break;
+      if (UF) {
+        F2.e[i][k] = ld_src<N, R, ADJF>(nf, i, k, S);
+        U2.e[k][i] = ld_link<R>(nu, k, i);
+      } else {
+        U2.e[i][k] = ld_link<R>(nu, i, k);
+        F2.e[k][i] = ld_src<N, R, ADJF>(nf, k, i, S);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < N; i++)
+#pragma unroll
+      for (int j = 0; j < N; j++) {
+        if (UF)
+          cfma(acc.e[i][j], u[i], f[j]);
+        else
+          cfma(acc.e[i][j], f[i], u[j]);
+      }
+  }
+  if (MORE) {
+    U = U2;
+    F = F2;
+  }
+}
+
+// The determinant terms from the pre-pass's traces (T_e = Tr U_e^-1 psi_e in
+// tr[e], Tr eta in tr[5]): detLtoS for the site component, detStoL for link B
+template <int N, typename R>
+SUSY_D void rl_det_site(Mat<N, R>& acc, const FopArgs<R>& a, const Site& c) {
+  const int S = a.g.S, s = c.s;
+  Cx<R> sum(0, 0);
+#pragma unroll 1
+  for (int b = 0; b < NUMLINK; b++) {
+    const int pb = nbr(a.g, c, ex(b), ey(b), ez(b), et(b));
+    const R bcb = bcf<R>(a.g, c, et(b));
+    const Cx<R> Tb = ldc<R>(a.trace + (size_t)b * S + s);
+#pragma unroll
+    for (int k = 1; k < NUMLINK; k++) {
+      const int e = b + k < NUMLINK ? b + k : b + k - NUMLINK;
+      const Cx<R> Te = ldc<R>(a.trace + (size_t)e * S + pb);
+      sum = sum + ldc<R>(a.pd + (size_t)(e * 5 + b) * S + s) * (Tb + bcb * Te);
+    }
+  }
+  const Cx<R> d = ((R)0.5 * a.G) * sum;
+#pragma unroll
+  for (int i = 0; i < N; i++) acc.e[i][i] = acc.e[i][i] + d;
+}
+template <int N, typename R>
+SUSY_D void rl_det_link(Mat<N, R>& acc, const FopArgs<R>& a, const Site& c, int B) {
+  const int S = a.g.S, s = c.s;
+  const typename CT<R>::T* te = a.trace + (size_t)5 * S;
+  const Cx<R> te0 = ldc<R>(te + s);
+  Cx<R> sum(0, 0);
+#pragma unroll
+  for (int k = 1; k < NUMLINK; k++) {
+    const int e = B + k < NUMLINK ? B + k : B + k - NUMLINK;
+    const int me = nbr(a.g, c, -ex(e), -ey(e), -ez(e), -et(e));
+    sum = sum + te0 * ldc<R>(a.pd + (size_t)(e * 5 + B) * S + s);
+    sum = sum + bcf<R>(a.g, c, -et(e)) * (ldc<R>(te + me) * ldc<R>(a.pd + (size_t)(B * 5 + e) * S + me));
+  }
+  const Cx<R> d = ((R)(-0.5) * a.G * a.eta_scale) * sum;
+  const typename CT<R>::T* pu = a.Uinv + (size_t)(B * N * N) * S + s;
+#pragma unroll
+  for (int i = 0; i < N; i++)
+#pragma unroll
+    for (int j = 0; j < N; j++) cfma(acc.e[i][j], d, ldc<R>(pu + (size_t)(i * N + j) * S));
+}
+
+template <int N, typename R, int SIGN, int MINB>
+__global__ void __launch_bounds__(RL_THREADS, MINB) fermion_op_rolling_kernel(FopArgs<R> a) {
+  typedef typename CT<R>::T T;
+  constexpr int NN = N * N;
+  constexpr bool AF = SIGN < 0;
+  if (a.skip && *a.skip) return;
+  const int comp = blockIdx.x % NTF;
+  const int s0 = (blockIdx.x / NTF) * RL_THREADS + threadIdx.x;
+  const int S = a.g.S;
+  const int s = min(s0, a.g.V - 1);   // lanes past the volume compute its last site
+  const int* tab = a.nbrtab + s;
+  const R pbc = (R)a.g.pbc;
+  unsigned bcm = 0;
+  {
+    const int t = s / (a.g.nx * a.g.ny * a.g.nz);
+#pragma unroll
+    for (int dt = -3; dt <= 3; dt++)
+      if (t + dt < 0 || t + dt > a.g.nt - 1) bcm |= 1u << (dt + 3);
+  }
+  auto link = [&](int C, int adj, int x) {
+    LinkPtr<R> u;
+    u.p = a.U + (size_t)(C * NN) * S + x;
+    u.si = adj ? S : N * S;
+    u.sj = adj ? N * S : S;
+    return u;
+  };
+  Mat<N, R> acc, U, F;
+  acc.zero();
+  RlTerm tm = c_rl[0][comp];
+  int xu2 = tab[(size_t)tm.ufu * S], xf2 = tab[(size_t)tm.dfu * S];
+  {
+    const LinkPtr<R> u = link(0, tm.adj, tab[(size_t)tm.uuf * S]);
+    const T* f = a.src + (size_t)(tm.k * NN) * S + tab[(size_t)tm.duf * S];
+#pragma unroll
+    for (int k = 0; k < N; k++)
+#pragma unroll
+      for (int i = 0; i < N; i++) {
+        U.e[i][k] = ld_link<R>(u, i, k);
+        F.e[k][i] = ld_src<N, R, AF>(f, k, i, S);
+      }
+  }
+  // the coefficient of a product, its BC factor and RESCALE's factor included
+  auto coef = [&](const RlTerm& q, float c, int bdt) {
+    return (R)c * bc_of<R>(bcm, bdt, pbc) * (q.k ? (R)1 : a.eta_scale);
+  };
+#pragma unroll 1
+  for (int C = 0; C < NUMLINK - 1; C++) {
+    const RlTerm tn = c_rl[C + 1][comp];
+    const int xu1 = tab[(size_t)tn.uuf * S], xf1 = tab[(size_t)tn.duf * S];
+    const R c1 = coef(tm, tm.cuf, tm.buf);
+    mac_roll<N, R, true, AF>(acc, c1, tm.adj ? -c1 : c1, U, F, link(C, tm.adj, xu2),
+                             a.src + (size_t)(tm.k * NN) * S + xf2, S);
+    xu2 = tab[(size_t)tn.ufu * S];
+    xf2 = tab[(size_t)tn.dfu * S];
+    const R c2 = coef(tm, tm.cfu, tm.bfu);
+    mac_roll<N, R, false, AF>(acc, c2, tm.adj ? -c2 : c2, U, F, link(C + 1, tn.adj, xu1),
+                              a.src + (size_t)(tn.k * NN) * S + xf1, S);
+    tm = tn;
+  }
+  {
+    const LinkPtr<R> u = link(NUMLINK - 1, tm.adj, xu2);
+    const T* f = a.src + (size_t)(tm.k * NN) * S + xf2;
+    const R c1 = coef(tm, tm.cuf, tm.buf), c2 = coef(tm, tm.cfu, tm.bfu);
+    mac_roll<N, R, true, AF>(acc, c1, tm.adj ? -c1 : c1, U, F, u, f, S);
+    mac_roll<N, R, false, AF, false>(acc, c2, tm.adj ? -c2 : c2, U, F, u, f, S);
+  }
+  const bool in = s0 < a.g.V;
+  double part = 0.0;
+  if (in) {
+    if (a.doG && comp <= NUMLINK) {
+      const Site c = site_of(a.g, s);
+      if (comp == 0)
+        rl_det_site(acc, a, c);
+      else
+        rl_det_link(acc, a, c, comp - 1);
+    }
+    if (comp == 0) eta_rescale(acc, a.eta_scale);
+    if (SIGN < 0) {
+      const Mat<N, R> m = acc;
+#pragma unroll
+      for (int i = 0; i < N; i++)
+#pragma unroll
+        for (int j = 0; j < N; j++) acc.e[i][j] = Cx<R>(-m.e[j][i].re, m.e[j][i].im);
+    }
+    if (a.add) {
+      const Mat<N, R> x = ldm<N, R>(a.add, comp, s, S);
+      axpy(acc, Cx<R>(a.addc, 0), x);
+      if (a.dot) part = rdot(x, acc);
+    }
+    stm<N, R>(a.dst, comp, s, S, acc);
+  }
+  if (a.dot) {
+    part = block_sum<RL_THREADS>(part);
+    if (threadIdx.x == 0) a.dot[blockIdx.x] = part;
+  }
+}
+
+template <int N, typename R, int MINB>
+static int launch_rolling(FopArgs<R> a, int sign, cudaStream_t st) {
+  const int nb = (a.g.V + RL_THREADS - 1) / RL_THREADS;
+  const dim3 nt(nb, NUMLINK + 1);
+  if (sign > 0) {
+    if (a.doG) count_launch(), k_det_traces<N, R, false><<<nt, RL_THREADS, 0, st>>>(a);
+    count_launch(), fermion_op_rolling_kernel<N, R, 1, MINB><<<nb * NTF, RL_THREADS, 0, st>>>(a);
+  } else {
+    if (a.doG) count_launch(), k_det_traces<N, R, true><<<nt, RL_THREADS, 0, st>>>(a);
+    count_launch(), fermion_op_rolling_kernel<N, R, -1, MINB><<<nb * NTF, RL_THREADS, 0, st>>>(a);
+  }
+  return nb * NTF;
+}
+
+// Resident blocks per SM: as many as hold a product's operands, the
+// accumulator and the addresses without spilling (80 / 64 registers for
+// NCOL 2, 128 / 80 for 3, 255 / 128 for 4, FP64 / FP32).  wide: a step fewer,
+// for lattices that do not fill the GPU anyway: more loads hoisted
+// (6^3x12 U(3) FP64 39.2 against 41.9 us; 12^3x24 293 against 263).
+template <typename R>
+int fermion_op_rolling(const FopArgs<R>& a, int N, int sign, bool wide, cudaStream_t st) {
+  constexpr bool D = sizeof(R) == 8;
+  switch (N) {
+    case 2: return wide ? launch_rolling<2, R, D ? 5 : 6>(a, sign, st) : launch_rolling<2, R, D ? 6 : 8>(a, sign, st);
+    case 3: return wide ? launch_rolling<3, R, D ? 3 : 5>(a, sign, st) : launch_rolling<3, R, D ? 4 : 6>(a, sign, st);
+    default: return launch_rolling<4, R, D ? 2 : 4>(a, sign, st);
+  }
+}
+
+template int fermion_op_rolling<double>(const FopArgs<double>&, int, int, bool, cudaStream_t);
+template int fermion_op_rolling<float>(const FopArgs<float>&, int, int, bool, cudaStream_t);
+
+}  // namespace susy

@@ -37,8 +37,7 @@ enum { P_UF = 0, P_FU = 1, P_FUD = 2, P_UDF = 3, NPAT = 4 };
 struct FTerm {
   int8_t kl, dl, kr, dr;   // components and displacement indices of the factors
   int8_t bcdt;
-  int8_t sl, sr;           // slots of dl, dr in the output's displacement list
-  int8_t pad;
+  int8_t pad[3];
   float coef;
 };
 
@@ -78,7 +77,7 @@ struct TermBuilder {
       }
     FTerm T;
     T.kl = kl; T.dl = dlv; T.kr = kr; T.dr = drv;
-    T.bcdt = bcdt; T.sl = T.sr = T.pad = 0;
+    T.bcdt = bcdt; T.pad[0] = T.pad[1] = T.pad[2] = 0;
     T.coef = (float)coef;
     terms[comp][pat].push_back(T);
   }
@@ -228,7 +227,8 @@ SUSY_D void det_ltos_rt(Mat<N, R>& acc, const FopArgs<R>& a, const Site& c) {
 
 // Every site's five detLtoS traces Tr(U_e^-1(x) src_{1+e}(x)) (the source
 // adjointed for D^dag), tr[e * S + x], summed as trace_ld sums them: the
-// pre-pass of FOP_SITE_MAJOR_TR.  One thread per (site, e), e = blockIdx.y:
+// pre-pass of FOP_SITE_MAJOR_TR and, with Tr src_0 in row e = 5, of
+// FOP_ROLLING.  One thread per (site, e), e = blockIdx.y:
 // one thread per site looping over e left too few loads in flight (the
 // pre-pass took ~25 us in FP64 at 12^3x24 U(3), for 63 MB; now 11.5 us).
 // Measured there (ncu, FP64): the operator kernel after it takes 147-154 us
@@ -245,6 +245,10 @@ __global__ void k_det_traces(FopArgs<R> a) {
   const int e = blockIdx.y;
   if (s >= a.g.V) return;
   const int S = a.g.S;
+  if (e == NUMLINK) {
+    stc<R>(a.trace + (size_t)e * S + s, ldtr<N, R, ADJ>(a.src, 0, s, S));
+    return;
+  }
   stc<R>(a.trace + (size_t)e * S + s, trace_ld<N, R, ADJ>(a.Uinv, e, s, a.src, 1 + e, s, S));
 }
 

@@ -85,8 +85,11 @@ struct MsBlockVecs {
 // 12^3x24 U(3): the FP64 optimum is the 128-register site-major kernel
 // (0.215 ms vs 0.260 uncapped; 102 registers: 0.256, 64: 0.59), the FP32 one
 // the 64-register component-major kernel (0.117 ms vs 0.135; 48: 0.166).
-// FOP_SITE_MAJOR_SHN / FOP_COMP_MAJOR_SHN: the _OCC kernels with each
-// block's neighbour indices preloaded into shared memory.
+// FOP_ROLLING / FOP_ROLLING_WIDE: table-driven by link direction, each
+// product's operands loaded while the one before it computes, the
+// determinant terms from the trace pre-pass (fermion_op_rolling.cu; without
+// the trace field they run as FOP_SITE_MAJOR_FRONT).  The autotuner's pick
+// from 8^4 on.
 // FOP_SITE_MAJOR_FRONT: site-major (FP64 4, FP32 8 blocks per SM) with the
 // site component's long blocks at the front of the grid.
 // FOP_GROUPED: one output component per warp over the same 32 sites, the
@@ -95,13 +98,12 @@ struct MsBlockVecs {
 // FOP_SITE_MAJOR_TR: FOP_SITE_MAJOR_FRONT after a pre-pass that writes
 // every site's five determinant traces, which the site component's detLtoS
 // term then reads instead of recomputing them at the site and its
-// neighbours (needs the handle's 5 S complex trace field; without one it
-// runs as FOP_SITE_MAJOR_FRONT).  The autotuner's pick in both precisions at
-// 12^3x24 U(3).
+// neighbours (needs the handle's 6 S complex trace field; without one it
+// runs as FOP_SITE_MAJOR_FRONT).
 enum { FOP_MAT = 0, FOP_MAT_CM = 1, FOP_ROWS = 2, FOP_COMPACT = 3, FOP_COMPACT_PF = 4,
        FOP_SITE_MAJOR_PP = 5, FOP_COMP_MAJOR_PP = 6, FOP_SITE_MAJOR = 7,
-       FOP_SITE_MAJOR_OCC = 8, FOP_COMP_MAJOR_OCC = 9, FOP_SITE_MAJOR_SHN = 10,
-       FOP_COMP_MAJOR_SHN = 11, FOP_SITE_MAJOR_FRONT = 12, FOP_GROUPED = 13,
+       FOP_SITE_MAJOR_OCC = 8, FOP_COMP_MAJOR_OCC = 9, FOP_ROLLING = 10,
+       FOP_ROLLING_WIDE = 11, FOP_SITE_MAJOR_FRONT = 12, FOP_GROUPED = 13,
        FOP_SITE_MAJOR_TR = 14, FOP_NVARIANTS = 15 };
 template <typename R>
 int fermion_op(const Geo& g, int N, const void* U, const void* Uinv, const void* pd,
@@ -112,6 +114,10 @@ template <typename R> struct FopArgs;
 template <typename R>
 int fermion_op_rows(const FopArgs<R>& a, int N, int sign, cudaStream_t st);
 int fop_partials(const Geo& g);
+template <typename R>
+int fermion_op_rolling(const FopArgs<R>& a, int N, int sign, bool wide, cudaStream_t st);
+// Its term table on the current device (upload_fop_terms)
+int upload_rolling_terms();
 template <typename R>
 int fermion_op_compact(const FopArgs<R>& a, int N, int sign, int variant, cudaStream_t st);
 // One application over n <= FOP_BATCH_MAX lattices of one NCOL in a single

@@ -28,7 +28,7 @@ struct susy_b200_lattice {
   void *U32 = nullptr, *Uinv32 = nullptr, *pd32 = nullptr;
   void* stage = nullptr;  // AoS staging buffer (one FP64 Twist_Fermion)
   int* nbrtab = nullptr;  // neighbour index table of the table-driven operator
-  void* trace[2] = {};    // determinant traces of FOP_SITE_MAJOR_TR (FP64, FP32);
+  void* trace[2] = {};    // determinant traces of the operator's pre-pass (FP64, FP32);
                           // each solver context owns its own
   void* ftrace = nullptr; // traces the fermion force's determinant terms read
   susy::MsState* ms = nullptr;

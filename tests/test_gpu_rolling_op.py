@@ -1,0 +1,39 @@
+"""The rolling-load operator kernels (fermion_op_rolling.cu) against the
+oracle around the edges of their 128-site tiles, for every NCOL, with and
+without the determinant terms and the mass term.  FP64: an entry is a sum of
+10 products of N terms and the determinant terms, two applications deep;
+FP32 the same in units of its rounding."""
+import numpy as np
+import pytest
+
+from oracle import susy_np as O
+from susy_b200 import Lattice, synth
+
+pytestmark = pytest.mark.gpu
+ROLLING = (10, 11)   # FOP_ROLLING, FOP_ROLLING_WIDE
+
+
+@pytest.mark.parametrize("dims,N,pbc,G,fmass", [
+    ((2, 2, 2, 2), 2, -1, 0.05, 0.0),      # 16 sites
+    ((2, 4, 4, 4), 3, 1, 0.05, 0.2),       # 128: one full tile
+    ((6, 2, 2, 6), 4, -1, 0.1, 0.0),       # 144: a tile and 16 sites
+    ((4, 4, 2, 8), 4, -1, 0.0, 0.3),       # 256, no determinant terms
+    ((4, 6, 2, 6), 2, -1, 0.05, 0.2)])     # 288
+def test_rolling_operator(dims, N, pbc, G, fmass):
+    U = synth.links(dims, N, 0.2, 7)
+    lat = Lattice(dims, N, pbc=pbc, lam=1.0, bmass=0.2, G=G, fmass=fmass)
+    lat.set_links(synth.to_ref(dims, U))
+    geo = O.Geometry(dims, pbc)
+    prm = O.Params(lam=1.0, bmass=0.2, G=G, fmass=fmass, N=N)
+    der = O.compute_derived(geo, prm, U)
+    src = synth.tf_source(dims, N, seed=21)
+    want = O.DSq(geo, prm, U, der, src)
+    for prec, tol in ((64, 1e-13), (32, 1e-5)):
+        for v in ROLLING:
+            lat.fop_variant(prec, v)
+            a64, a, b = lat.tf(64), lat.tf(prec), lat.tf(prec)
+            a64.upload(synth.to_ref(dims, src))
+            lat.dev_convert(a64, a)
+            lat.dev_DSq(a, b)
+            got = synth.from_ref(dims, b.download(), 16, N)
+            assert np.abs(got - want).max() <= tol * np.abs(want).max()
