@@ -101,7 +101,9 @@ FopArgs<R> batch_fop_args(susy_b200_lattice* h, const void* src, void* dst, cons
   a.nsb = 0;
   a.nbrtab = h->nbrtab;
   a.eta_scale = (R)(h->rescale ? 2.0 : 1.0);
-  a.trace = nullptr;
+  a.trace = (T*)h->trace[f64 ? 0 : 1];
+  a.trace_out = nullptr;
+  a.traces_ready = 0;
   return a;
 }
 template FopArgs<double> batch_fop_args<double>(susy_b200_lattice*, const void*, void*,
@@ -143,7 +145,7 @@ static int dsq_batch(susy_b200_lattice* const* hs, const void* const* src, void*
   std::vector<FopArgs<R>> a(n);
   for (int i = 0; i < n; i++)
     a[i] = batch_fop_args<R>(hs[i], src[i], tmp[i], nullptr, 0.0, nullptr, nullptr);
-  int rc = fermion_op_batch<R>(a.data(), n, hs[0]->N, 1, sms, st) < 0 ? SUSY_B200_EINVAL : 0;
+  int rc = fermion_op_batch<R>(a.data(), n, hs[0]->N, 1, FOP_FIRST, sms, st) < 0 ? SUSY_B200_EINVAL : 0;
   if (!rc) {
     for (int i = 0; i < n; i++) {
       const double fm = hs[i]->prm.fmass;
@@ -151,7 +153,7 @@ static int dsq_batch(susy_b200_lattice* const* hs, const void* const* src, void*
       a[i] = batch_fop_args<R>(hs[i], tmp[i], dst[i], fm2 != 0.0 ? src[i] : nullptr, fm2,
                                nullptr, nullptr);
     }
-    rc = fermion_op_batch<R>(a.data(), n, hs[0]->N, -1, sms, st) < 0 ? SUSY_B200_EINVAL : 0;
+    rc = fermion_op_batch<R>(a.data(), n, hs[0]->N, -1, FOP_SECOND, sms, st) < 0 ? SUSY_B200_EINVAL : 0;
   }
   for (cudaStream_t o : others)
     if (!order(st, o) && !rc) rc = SUSY_B200_ECUDA;

@@ -126,14 +126,15 @@ void refresh_low(susy_b200_lattice* h) {
 // FOP_COMPACT on) apply the factor; a variant below them is replaced by
 // FOP_SITE_MAJOR_OCC.
 static int launch_variant(susy_b200_lattice* h, const void* src, void* dst, int sign, int prec,
-                          const void* add, double addc, double* dot, const int* skip, int v) {
+                          const void* add, double addc, double* dot, const int* skip, int v,
+                          int chain) {
   const double es = h->rescale ? 2.0 : 1.0;
   if (h->rescale && v < FOP_COMPACT) v = FOP_SITE_MAJOR_OCC;
   if (prec == 64)
     return fermion_op<double>(h->g, h->N, h->U, h->Uinv, h->pd, src, dst, sign, h->G, add, addc,
-                              dot, skip, v, h->nbrtab, h->stream, es, h->trace[0]);
+                              dot, skip, v, h->nbrtab, h->stream, es, h->trace[0], chain);
   return fermion_op<float>(h->g, h->N, h->U32, h->Uinv32, h->pd32, src, dst, sign, h->G, add,
-                           addc, dot, skip, v, h->nbrtab, h->stream, es, h->trace[1]);
+                           addc, dot, skip, v, h->nbrtab, h->stream, es, h->trace[1], chain);
 }
 
 // Project-written autotuner: time one D^dag D with every kernel variant on
@@ -152,11 +153,11 @@ int autotune_fop(susy_b200_lattice* h, int prec) {
   float best = 1e30f;
   int bestv = h->rescale ? FOP_SITE_MAJOR_OCC : FOP_MAT;
   for (int v = h->rescale ? FOP_COMPACT : 0; v < FOP_NVARIANTS; v++) {
-    launch_variant(h, a, b, 1, prec, nullptr, 0.0, nullptr, nullptr, v);
+    launch_variant(h, a, b, 1, prec, nullptr, 0.0, nullptr, nullptr, v, FOP_ALONE);
     cudaEventRecord(e0, h->stream);
     for (int r = 0; r < 3; r++) {
-      launch_variant(h, a, b, 1, prec, nullptr, 0.0, nullptr, nullptr, v);
-      launch_variant(h, b, a, -1, prec, nullptr, 0.0, nullptr, nullptr, v);
+      launch_variant(h, a, b, 1, prec, nullptr, 0.0, nullptr, nullptr, v, FOP_FIRST);
+      launch_variant(h, b, a, -1, prec, nullptr, 0.0, nullptr, nullptr, v, FOP_SECOND);
     }
     cudaEventRecord(e1, h->stream);
     cudaEventSynchronize(e1);
@@ -175,10 +176,10 @@ int autotune_fop(susy_b200_lattice* h, int prec) {
 }
 
 int dev_fop(susy_b200_lattice* h, const void* src, void* dst, int sign, int prec,
-            const void* add, double addc, double* dot, const int* skip) {
+            const void* add, double addc, double* dot, const int* skip, int chain) {
   const int pi = prec == 64 ? 0 : 1;
   if (h->fop_variant[pi] < 0) autotune_fop(h, prec);
-  return launch_variant(h, src, dst, sign, prec, add, addc, dot, skip, h->fop_variant[pi]);
+  return launch_variant(h, src, dst, sign, prec, add, addc, dot, skip, h->fop_variant[pi], chain);
 }
 
 void* scratch_tf(susy_b200_lattice* h, int which, int prec) {
@@ -236,8 +237,8 @@ susy_b200_lattice* solver_shadow(susy_b200_lattice* h) {
     }
     c->stream = c->own_stream;
     c->ms = (MsState*)dalloc(c, sizeof(MsState));
-    c->trace[0] = dalloc(c, 6 * c->g.S * sizeof(double2));
-    c->trace[1] = dalloc(c, 6 * c->g.S * sizeof(float2));
+    c->trace[0] = dalloc(c, 12 * c->g.S * sizeof(double2));
+    c->trace[1] = dalloc(c, 12 * c->g.S * sizeof(float2));
     if (!c->ms || !c->trace[0] || !c->trace[1]) {
       susy_b200_destroy(c);
       return nullptr;
@@ -315,8 +316,8 @@ susy_b200_lattice* susy_b200_create(const susy_b200_params* p) {
   h->stage = dalloc(h, (size_t)h->g.V * NTF * mat_c(h) * 2 * sizeof(double));
   h->ms = (MsState*)dalloc(h, sizeof(MsState));
   h->nbrtab = (int*)dalloc(h, (size_t)fop_ndisp() * h->g.S * sizeof(int));
-  h->trace[0] = dalloc(h, 6 * h->g.S * sizeof(double2));
-  h->trace[1] = dalloc(h, 6 * h->g.S * sizeof(float2));
+  h->trace[0] = dalloc(h, 12 * h->g.S * sizeof(double2));
+  h->trace[1] = dalloc(h, 12 * h->g.S * sizeof(float2));
   if (h->nbrtab) build_nbr_table(h->g, h->nbrtab, h->stream);
   if (h->err) {
     susy_b200_destroy(h);
@@ -649,8 +650,8 @@ int susy_b200_dev_DSq(susy_b200_lattice* h, const void* src, void* dst, int prec
   void* tmp = scratch_tf(h, 0, prec);
   if (!tmp) return SUSY_B200_ENOMEM;
   const double fm2 = h->prm.fmass > 1e-8 ? h->prm.fmass * h->prm.fmass : 0.0;
-  dev_fop(h, src, tmp, 1, prec, nullptr, 0.0, nullptr, nullptr);
-  dev_fop(h, tmp, dst, -1, prec, fm2 != 0.0 ? src : nullptr, fm2, nullptr, nullptr);
+  dev_fop(h, src, tmp, 1, prec, nullptr, 0.0, nullptr, nullptr, FOP_FIRST);
+  dev_fop(h, tmp, dst, -1, prec, fm2 != 0.0 ? src : nullptr, fm2, nullptr, nullptr, FOP_SECOND);
   return ck(h, cudaGetLastError()) ? SUSY_B200_OK : SUSY_B200_ECUDA;
 }
 

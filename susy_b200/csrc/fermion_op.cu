@@ -259,7 +259,7 @@ template <typename R>
 int fermion_op(const Geo& g, int N, const void* U, const void* Uinv, const void* pd,
                 const void* src, void* dst, int sign, double G, const void* add,
                 double addc, double* dot, const int* skip, int variant, const int* nbrtab,
-                cudaStream_t st, double eta_scale, void* trace) {
+                cudaStream_t st, double eta_scale, void* trace, int chain) {
   typedef typename CT<R>::T T;
   FopArgs<R> a;
   a.g = g;
@@ -277,11 +277,18 @@ int fermion_op(const Geo& g, int N, const void* U, const void* Uinv, const void*
   a.nbrtab = nbrtab;
   a.eta_scale = (R)eta_scale;
   a.trace = (T*)trace;
+  a.trace_out = nullptr;
+  a.traces_ready = 0;
   if (variant == FOP_SITE_MAJOR_TR && !trace) variant = FOP_SITE_MAJOR_FRONT;
   if (variant == FOP_ROWS) return fermion_op_rows<R>(a, N, sign, st);
   const bool rolling = variant == FOP_ROLLING || variant == FOP_ROLLING_WIDE;
   if (rolling && !trace) variant = FOP_SITE_MAJOR_FRONT;
-  else if (rolling) return fermion_op_rolling<R>(a, N, sign, variant == FOP_ROLLING_WIDE, st);
+  if (rolling && trace && a.doG && chain == FOP_FIRST) a.trace_out = (T*)trace + 6 * (size_t)g.S;
+  if (rolling && trace && a.doG && chain == FOP_SECOND) {
+    a.trace = (T*)trace + 6 * (size_t)g.S;
+    a.traces_ready = 1;
+  }
+  if (rolling && trace) return fermion_op_rolling<R>(a, N, sign, variant == FOP_ROLLING_WIDE, st);
   if (variant >= FOP_COMPACT) return fermion_op_compact<R>(a, N, sign, variant, st);
   a.comp_major = variant == FOP_MAT_CM;
   switch (N) {
@@ -294,10 +301,10 @@ int fermion_op(const Geo& g, int N, const void* U, const void* Uinv, const void*
 template int fermion_op<double>(const Geo&, int, const void*, const void*, const void*,
                                  const void*, void*, int, double, const void*, double,
                                  double*, const int*, int, const int*, cudaStream_t, double,
-                                 void*);
+                                 void*, int);
 template int fermion_op<float>(const Geo&, int, const void*, const void*, const void*,
                                 const void*, void*, int, double, const void*, double,
                                 double*, const int*, int, const int*, cudaStream_t, double,
-                                void*);
+                                void*, int);
 
 }  // namespace susy

@@ -179,16 +179,15 @@ SUSY_D void rl_det_link(Mat<N, R>& acc, const FopArgs<R>& a, const Site& c, int 
     for (int j = 0; j < N; j++) cfma(acc.e[i][j], d, ldc<R>(pu + (size_t)(i * N + j) * S));
 }
 
-template <int N, typename R, int SIGN, int MINB>
-__global__ void __launch_bounds__(RL_THREADS, MINB) fermion_op_rolling_kernel(FopArgs<R> a) {
+// Output component comp at site s0 (lanes past the volume compute and drop its
+// last site); returns the site's share of the epilogue's inner product
+template <int N, typename R, int SIGN>
+SUSY_D double rl_site(const FopArgs<R>& a, int comp, int s0) {
   typedef typename CT<R>::T T;
   constexpr int NN = N * N;
   constexpr bool AF = SIGN < 0;
-  if (a.skip && *a.skip) return;
-  const int comp = blockIdx.x % NTF;
-  const int s0 = (blockIdx.x / NTF) * RL_THREADS + threadIdx.x;
   const int S = a.g.S;
-  const int s = min(s0, a.g.V - 1);   // lanes past the volume compute its last site
+  const int s = min(s0, a.g.V - 1);
   const int* tab = a.nbrtab + s;
   const R pbc = (R)a.g.pbc;
   unsigned bcm = 0;
@@ -269,7 +268,31 @@ __global__ void __launch_bounds__(RL_THREADS, MINB) fermion_op_rolling_kernel(Fo
       if (a.dot) part = rdot(x, acc);
     }
     stm<N, R>(a.dst, comp, s, S, acc);
+    if (SIGN > 0 && a.trace_out && comp <= NUMLINK) {
+      // the traces of this result's adjoint, the source of the D^dag to come,
+      // summed as k_det_traces sums them
+      Cx<R> t(0, 0);
+      if (comp == 0) {
+        t = conj(trace(acc));
+      } else {
+        const T* pu = a.Uinv + (size_t)((comp - 1) * NN) * S + s;
+#pragma unroll
+        for (int i = 0; i < N; i++)
+#pragma unroll
+          for (int j = 0; j < N; j++)
+            t = t + ldc<R>(pu + (size_t)(i * N + j) * S) * conj(acc.e[i][j]);
+      }
+      stc<R>(a.trace_out + (size_t)(comp == 0 ? NUMLINK : comp - 1) * S + s, t);
+    }
   }
+  return part;
+}
+
+template <int N, typename R, int SIGN, int MINB>
+__global__ void __launch_bounds__(RL_THREADS, MINB) fermion_op_rolling_kernel(FopArgs<R> a) {
+  if (a.skip && *a.skip) return;
+  double part = rl_site<N, R, SIGN>(a, blockIdx.x % NTF,
+                                    (blockIdx.x / NTF) * RL_THREADS + threadIdx.x);
   if (a.dot) {
     part = block_sum<RL_THREADS>(part);
     if (threadIdx.x == 0) a.dot[blockIdx.x] = part;
@@ -281,10 +304,10 @@ static int launch_rolling(FopArgs<R> a, int sign, cudaStream_t st) {
   const int nb = (a.g.V + RL_THREADS - 1) / RL_THREADS;
   const dim3 nt(nb, NUMLINK + 1);
   if (sign > 0) {
-    if (a.doG) count_launch(), k_det_traces<N, R, false><<<nt, RL_THREADS, 0, st>>>(a);
+    if (a.doG && !a.traces_ready) count_launch(), k_det_traces<N, R, false><<<nt, RL_THREADS, 0, st>>>(a);
     count_launch(), fermion_op_rolling_kernel<N, R, 1, MINB><<<nb * NTF, RL_THREADS, 0, st>>>(a);
   } else {
-    if (a.doG) count_launch(), k_det_traces<N, R, true><<<nt, RL_THREADS, 0, st>>>(a);
+    if (a.doG && !a.traces_ready) count_launch(), k_det_traces<N, R, true><<<nt, RL_THREADS, 0, st>>>(a);
     count_launch(), fermion_op_rolling_kernel<N, R, -1, MINB><<<nb * NTF, RL_THREADS, 0, st>>>(a);
   }
   return nb * NTF;
@@ -307,5 +330,117 @@ int fermion_op_rolling(const FopArgs<R>& a, int N, int sign, bool wide, cudaStre
 
 template int fermion_op_rolling<double>(const FopArgs<double>&, int, int, bool, cudaStream_t);
 template int fermion_op_rolling<float>(const FopArgs<float>&, int, int, bool, cudaStream_t);
+
+// ---------------------------------------------------------------------------
+// One operator application over many independent lattices of one NCOL in a
+// single persistent launch (susy_b200_DSq_batch).  Item w of the work table is
+// output component w % 16 of global tile w / 16; a global tile belongs to the
+// lattice whose tile range holds it.  Each lattice keeps its own geometry,
+// fields, couplings and neighbour table (FopArgs), all passed in the kernel's
+// parameter space, so the launch needs no device memory of its own.  The grid
+// is resident-sized (blocks per SM x SMs) and every block walks the table
+// with a stride of the grid, so lattices of 256 sites and of 8192 fill the
+// GPU together.  An item is the rolling kernel's block, so each lattice gets
+// the same result as its own launch.  A lattice whose skip flag is set (its
+// solve has finished) contributes no work; with a dot field, lattice i's item
+// (tile t, component k) writes its block's share of the epilogue's inner
+// product to dot[k * tiles_i + t] (16 tiles_i partials per lattice).
+template <typename R>
+struct FopBatch {
+  int n;                          // lattices
+  int tiles;                      // 128-site tiles of all lattices
+  int start[FOP_BATCH_MAX + 1];   // first global tile of lattice i
+  FopArgs<R> a[FOP_BATCH_MAX];
+};
+// kernel parameters may take up to 32764 bytes (CUDA 12.1 and later)
+static_assert(sizeof(FopBatch<double>) <= 32000, "batch arguments exceed the parameter space");
+
+// Largest i < n with start[i] <= t
+SUSY_D int batch_lattice(const int* start, int n, int t) {
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (start[mid] <= t)
+      lo = mid;
+    else
+      hi = mid - 1;
+  }
+  return lo;
+}
+
+template <int N, typename R, int SIGN, int MINB>
+__global__ void __launch_bounds__(RL_THREADS, MINB)
+fermion_op_batch_kernel(const __grid_constant__ FopBatch<R> B) {
+  const int total = NTF * B.tiles;
+#pragma unroll 1
+  for (int w = blockIdx.x; w < total; w += gridDim.x) {
+    const int gt = w / NTF, comp = w % NTF;
+    const int i = batch_lattice(B.start, B.n, gt);
+    const FopArgs<R>& a = B.a[i];
+    if (a.skip && *a.skip) continue;   // the whole block: one lattice per item
+    const int tile = gt - B.start[i];
+    double part = rl_site<N, R, SIGN>(a, comp, tile * RL_THREADS + threadIdx.x);
+    if (a.dot) {
+      part = block_sum<RL_THREADS>(part);
+      if (threadIdx.x == 0) a.dot[comp * (B.start[i + 1] - B.start[i]) + tile] = part;
+      __syncthreads();   // block_sum's shared words are reused by the next item
+    }
+  }
+}
+
+// The trace pre-pass of every lattice: block (gt, e)
+template <int N, typename R, bool ADJ>
+__global__ void k_det_traces_batch(const __grid_constant__ FopBatch<R> B) {
+  const int i = batch_lattice(B.start, B.n, blockIdx.x);
+  const FopArgs<R>& a = B.a[i];
+  if (!a.doG || (a.skip && *a.skip)) return;
+  det_traces_site<N, R, ADJ>(a, (blockIdx.x - B.start[i]) * RL_THREADS + threadIdx.x, blockIdx.y);
+}
+
+template <int N, typename R, int MINB>
+static void launch_batch(const FopBatch<R>& B, int sign, bool traces, int sms, cudaStream_t st) {
+  const int grid = NTF * B.tiles < MINB * sms ? NTF * B.tiles : MINB * sms;
+  const dim3 nt(B.tiles, NUMLINK + 1);
+  if (sign > 0) {
+    if (traces) count_launch(), k_det_traces_batch<N, R, false><<<nt, RL_THREADS, 0, st>>>(B);
+    count_launch(), fermion_op_batch_kernel<N, R, 1, MINB><<<grid, RL_THREADS, 0, st>>>(B);
+  } else {
+    if (traces) count_launch(), k_det_traces_batch<N, R, true><<<nt, RL_THREADS, 0, st>>>(B);
+    count_launch(), fermion_op_batch_kernel<N, R, -1, MINB><<<grid, RL_THREADS, 0, st>>>(B);
+  }
+}
+
+template <typename R>
+int fermion_op_batch(const FopArgs<R>* args, int n, int N, int sign, int chain, int sms,
+                     cudaStream_t st) {
+  if (n < 1 || n > FOP_BATCH_MAX || N < 2 || N > 4 || sms < 1) return -1;
+  FopBatch<R> B;
+  B.n = n;
+  long t = 0;
+  bool traces = false;
+  for (int i = 0; i < n; i++) {
+    FopArgs<R>& a = B.a[i];
+    a = args[i];
+    if (!a.trace) return -1;
+    if (chain == FOP_FIRST && a.doG) a.trace_out = a.trace + 6 * (size_t)a.g.S;
+    if (chain == FOP_SECOND) a.trace += 6 * (size_t)a.g.S;
+    traces = traces || (a.doG && chain != FOP_SECOND);
+    B.start[i] = (int)t;
+    t += (a.g.V + RL_THREADS - 1) / RL_THREADS;
+  }
+  if (NTF * t > 0x7fffffffL) return -1;
+  B.tiles = (int)t;
+  B.start[n] = (int)t;
+  constexpr bool D = sizeof(R) == 8;
+  switch (N) {
+    case 2: launch_batch<2, R, D ? 6 : 8>(B, sign, traces, sms, st); break;
+    case 3: launch_batch<3, R, D ? 4 : 6>(B, sign, traces, sms, st); break;
+    default: launch_batch<4, R, D ? 2 : 4>(B, sign, traces, sms, st); break;
+  }
+  return (int)(NTF * t);
+}
+
+template int fermion_op_batch<double>(const FopArgs<double>*, int, int, int, int, int, cudaStream_t);
+template int fermion_op_batch<float>(const FopArgs<float>*, int, int, int, int, int, cudaStream_t);
 
 }  // namespace susy

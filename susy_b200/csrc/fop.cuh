@@ -26,6 +26,9 @@ struct FopArgs {
                       // input and output doubled, utilities.c:795,841), else 1
   T* trace;           // the five traces Tr(U_e^-1 src_{1+e}) of every site and
                       // Tr src_0, [e][S] (written by the pre-pass k_det_traces)
+  T* trace_out;       // rolling kernels, D only: the same traces of dst as D^dag
+                      // reads them, or null
+  int traces_ready;   // rolling kernels: trace is already that of src
 };
 
 constexpr int FOP_THREADS = 128;

@@ -239,17 +239,17 @@ SUSY_D void det_ltos_rt(Mat<N, R>& acc, const FopArgs<R>& a, const Site& c) {
 // without it, and 0.171 / 0.101 with the trace pre-pass but the plain
 // site-major block order.
 template <int N, typename R, bool ADJ>
-__global__ void k_det_traces(FopArgs<R> a) {
-  if (a.skip && *a.skip) return;
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  const int e = blockIdx.y;
+SUSY_D void det_traces_site(const FopArgs<R>& a, int s, int e) {
   if (s >= a.g.V) return;
   const int S = a.g.S;
-  if (e == NUMLINK) {
-    stc<R>(a.trace + (size_t)e * S + s, ldtr<N, R, ADJ>(a.src, 0, s, S));
-    return;
-  }
-  stc<R>(a.trace + (size_t)e * S + s, trace_ld<N, R, ADJ>(a.Uinv, e, s, a.src, 1 + e, s, S));
+  const Cx<R> t = e == NUMLINK ? ldtr<N, R, ADJ>(a.src, 0, s, S)
+                               : trace_ld<N, R, ADJ>(a.Uinv, e, s, a.src, 1 + e, s, S);
+  stc<R>(a.trace + (size_t)e * S + s, t);
+}
+template <int N, typename R, bool ADJ>
+__global__ void k_det_traces(FopArgs<R> a) {
+  if (a.skip && *a.skip) return;
+  det_traces_site<N, R, ADJ>(a, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y);
 }
 
 // detLtoS from the pre-pass's traces: the sums of det_ltos_rt in the same

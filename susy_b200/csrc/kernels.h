@@ -98,18 +98,22 @@ struct MsBlockVecs {
 // FOP_SITE_MAJOR_TR: FOP_SITE_MAJOR_FRONT after a pre-pass that writes
 // every site's five determinant traces, which the site component's detLtoS
 // term then reads instead of recomputing them at the site and its
-// neighbours (needs the handle's 6 S complex trace field; without one it
+// neighbours (needs the handle's trace field; without one it
 // runs as FOP_SITE_MAJOR_FRONT).
 enum { FOP_MAT = 0, FOP_MAT_CM = 1, FOP_ROWS = 2, FOP_COMPACT = 3, FOP_COMPACT_PF = 4,
        FOP_SITE_MAJOR_PP = 5, FOP_COMP_MAJOR_PP = 6, FOP_SITE_MAJOR = 7,
        FOP_SITE_MAJOR_OCC = 8, FOP_COMP_MAJOR_OCC = 9, FOP_ROLLING = 10,
        FOP_ROLLING_WIDE = 11, FOP_SITE_MAJOR_FRONT = 12, FOP_GROUPED = 13,
        FOP_SITE_MAJOR_TR = 14, FOP_NVARIANTS = 15 };
+// D and the D^dag that follows it on D's result, with nothing between them on
+// the context: the rolling kernels' D then writes the traces that D^dag reads
+// (the second 6 S complex of the trace field), saving that pre-pass.
+enum { FOP_ALONE = 0, FOP_FIRST = 1, FOP_SECOND = 2 };
 template <typename R>
 int fermion_op(const Geo& g, int N, const void* U, const void* Uinv, const void* pd,
                 const void* src, void* dst, int sign, double G, const void* add, double addc,
                 double* dot, const int* skip, int variant, const int* nbrtab, cudaStream_t st,
-                double eta_scale = 1.0, void* trace = nullptr);
+                double eta_scale = 1.0, void* trace = nullptr, int chain = FOP_ALONE);
 template <typename R> struct FopArgs;
 template <typename R>
 int fermion_op_rows(const FopArgs<R>& a, int N, int sign, cudaStream_t st);
@@ -121,12 +125,14 @@ int upload_rolling_terms();
 template <typename R>
 int fermion_op_compact(const FopArgs<R>& a, int N, int sign, int variant, cudaStream_t st);
 // One application over n <= FOP_BATCH_MAX lattices of one NCOL in a single
-// persistent launch over a work table (fermion_op_compact.cu); the args
-// carry no trace; a lattice's dot field receives 16 ceil(V / 128) partials.
-// Returns the work items, < 0 on bad input.
+// persistent launch over a work table (fermion_op_rolling.cu), after one
+// trace pre-pass for all of them (chain as in fermion_op); a lattice's dot
+// field receives 16 ceil(V / 128) partials.  Returns the work items, < 0 on
+// bad input.
 constexpr int FOP_BATCH_MAX = 64;
 template <typename R>
-int fermion_op_batch(const FopArgs<R>* args, int n, int N, int sign, int sms, cudaStream_t st);
+int fermion_op_batch(const FopArgs<R>* args, int n, int N, int sign, int chain, int sms,
+                     cudaStream_t st);
 int upload_fop_terms(int device, cudaStream_t st);
 int fop_ndisp();
 void build_nbr_table(const Geo& g, int* tab, cudaStream_t st);

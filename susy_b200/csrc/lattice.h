@@ -85,7 +85,8 @@ int download_links(susy_b200_lattice* h, const void* dev, double* host, size_t s
 int refresh_derived(susy_b200_lattice* h);
 void refresh_low(susy_b200_lattice* h);
 int dev_fop(susy_b200_lattice* h, const void* src, void* dst, int sign, int prec,
-            const void* add, double addc, double* dot, const int* skip);
+            const void* add, double addc, double* dot, const int* skip,
+            int chain = FOP_ALONE);
 int autotune_fop(susy_b200_lattice* h, int prec);
 void* scratch_tf(susy_b200_lattice* h, int which, int prec);
 double* partials(susy_b200_lattice* h, int which);

@@ -89,8 +89,9 @@ static int ms_run(susy_b200_lattice* h, const void* src, void* const* psim, int 
   int launched = 0;
   for (;;) {
     for (int k = 0; k < chunk; k++) {
-      dev_fop(h, p0, tmp, 1, pv, nullptr, 0.0, nullptr, skip);
-      const int np_fop = dev_fop(h, tmp, mp, -1, pv, p0, fm2 + shift[0], part0, skip);
+      dev_fop(h, p0, tmp, 1, pv, nullptr, 0.0, nullptr, skip, FOP_FIRST);
+      const int np_fop = dev_fop(h, tmp, mp, -1, pv, p0, fm2 + shift[0], part0, skip,
+                                 FOP_SECOND);
       ms_scalars1(h->ms, part0, np_fop, s);
       ms_update_fused(h->ms, v, pv, px, n, part1, s);
       ms_scalars2(h->ms, part1, np_vec, s);
@@ -195,8 +196,8 @@ static int ms_run_batch(susy_b200_lattice* const* hs, int nl, const void* const*
   int launched = 0;
   for (;;) {
     for (int k = 0; k < chunk && !rc; k++) {
-      if (fermion_op_batch<double>(aD.data(), nl, N, 1, sms, st) < 0 ||
-          fermion_op_batch<double>(aDd.data(), nl, N, -1, sms, st) < 0)
+      if (fermion_op_batch<double>(aD.data(), nl, N, 1, FOP_FIRST, sms, st) < 0 ||
+          fermion_op_batch<double>(aDd.data(), nl, N, -1, FOP_SECOND, sms, st) < 0)
         rc = SUSY_B200_EINVAL;
       ms_batch_scalars1(dL, nl, st);
       ms_batch_update_fused(dL, nl, vtot, st);
@@ -393,11 +394,11 @@ static int ms_run_block(susy_b200_lattice* h, const void* src, void* const* psim
     for (int k = 0; k < chunk; k++) {
       int np_fop;
       if (fp32_op) {
-        dev_fop(h, p0_32, tmp32, 1, 32, nullptr, 0.0, nullptr, skip);
-        np_fop = dev_fop(h, tmp32, mp32, -1, 32, p0_32, fm2 + shift[0], part0, skip);
+        dev_fop(h, p0_32, tmp32, 1, 32, nullptr, 0.0, nullptr, skip, FOP_FIRST);
+        np_fop = dev_fop(h, tmp32, mp32, -1, 32, p0_32, fm2 + shift[0], part0, skip, FOP_SECOND);
       } else {
-        dev_fop(h, p0, tmp, 1, 64, nullptr, 0.0, nullptr, skip);
-        np_fop = dev_fop(h, tmp, mp, -1, 64, p0, fm2 + shift[0], part0, skip);
+        dev_fop(h, p0, tmp, 1, 64, nullptr, 0.0, nullptr, skip, FOP_FIRST);
+        np_fop = dev_fop(h, tmp, mp, -1, 64, p0, fm2 + shift[0], part0, skip, FOP_SECOND);
       }
       ms_scalars1(h->ms, part0, np_fop, s);
       msb_update_r(h->ms, v, n, part1, fp32_op, s);
@@ -530,8 +531,8 @@ static double true_residual(susy_b200_lattice* h, const void* b, const void* x, 
   void* t = scratch_tf(h, 0, 64);
   void* ax = refine_field(h, 2, 64);
   double* part = partials(h, 2);
-  dev_fop(h, x, t, 1, 64, nullptr, 0.0, nullptr, nullptr);
-  dev_fop(h, t, ax, -1, 64, x, fm2 + sigma, nullptr, nullptr);
+  dev_fop(h, x, t, 1, 64, nullptr, 0.0, nullptr, nullptr, FOP_FIRST);
+  dev_fop(h, t, ax, -1, 64, x, fm2 + sigma, nullptr, nullptr, FOP_SECOND);
   const int nb = residual_partials(tf_complex(h), b, ax, r64, r32, part, h->stream);
   return host_sum(h, part, nb, 0);
 }
@@ -632,8 +633,8 @@ static int fcg_refine(susy_b200_lattice* h, susy_b200_net* net, const void* b, v
     return host_sum(h, part, nb, 0);
   };
   auto apply_A = [&](const void* in, void* out) {
-    dev_fop(h, in, t, 1, 64, nullptr, 0.0, nullptr, nullptr);
-    dev_fop(h, t, out, -1, 64, in, fm2 + sigma, nullptr, nullptr);
+    dev_fop(h, in, t, 1, 64, nullptr, 0.0, nullptr, nullptr, FOP_FIRST);
+    dev_fop(h, t, out, -1, 64, in, fm2 + sigma, nullptr, nullptr, FOP_SECOND);
   };
   auto precond = [&](const void* in, void* out) -> int {
     if (net) return net_apply(net, in, out);
