@@ -127,6 +127,39 @@ __global__ void k_ms_scalars1(MsState* st, const double* partials, int np) {
   scalars1_block(st, partials, np, sh);
 }
 
+// Shift j's combination coefficients of a block of L iterations (see the
+// blocked update below), from the history this thread recorded.  Once per
+// block here; each CTA of the block pass deriving them again cost it 2 us.
+SUSY_D void block_coefs(MsState* st, int j, int L) {
+  // c_t and d_{t,s} for t = 0..L, s = 1..t (d indexed s-1)
+  double c = 1.0, d[MS_BLK];
+  double x0 = 0.0, xr[MS_BLK];
+#pragma unroll
+  for (int q = 0; q < MS_BLK; q++) d[q] = xr[q] = 0.0;
+  for (int t = 0; t < L; t++) {
+    const double b = st->hb[t][j], z = st->hz[t][j], a = st->ha[t][j];
+    // psi -= b_t p(k + t)
+    x0 += b * c;
+#pragma unroll
+    for (int q = 0; q < MS_BLK; q++)
+      if (q < t) xr[q] += b * d[q];
+    // p(k + t + 1) = z_t R_{t+1} + a_t p(k + t)
+    c *= a;
+#pragma unroll
+    for (int q = 0; q < MS_BLK; q++) {
+      if (q < t) d[q] *= a;
+      if (q == t) d[q] = z;
+    }
+  }
+  st->cx0[j] = x0;
+  st->cp0[j] = c;
+#pragma unroll
+  for (int q = 0; q < MS_BLK; q++) {
+    st->cxr[q][j] = xr[q];
+    st->cpr[q][j] = d[q];
+  }
+}
+
 // The scalar recurrences after the residual update, run by one block of ST
 // threads (thread j: shift j): its own kernel, or the last block of the
 // fused residual update (partials read from L2: other blocks wrote them)
@@ -174,10 +207,12 @@ SUSY_D void scalars2_block(MsState* st, const double* partials, int np, double* 
       st->zeta_i[j] = zp;
     }
   }
+  const bool stop = rsqnew <= st->rsqstop || st->iter >= st->maxcg;
+  if (t >= 0 && (t + 1 == MS_BLK || stop) && mine) block_coefs(st, j, t + 1);
   if (j == 0) {
     if (t >= 0) st->blk_len = t + 1;
     st->rsq = rsqnew;
-    st->skip = (rsqnew <= st->rsqstop || st->iter >= st->maxcg) ? 1 : 0;
+    st->skip = stop ? 1 : 0;
   }
 }
 
@@ -491,9 +526,11 @@ template <> SUSY_D double2 rnd2<float2>(double2 v) {
   return make_double2((double)(float)v.x, (double)(float)v.y);
 }
 
+// blk of nblk blocks, grid-stride: few blocks, so the last one sums few
+// partials
 template <typename MT, typename RT>
-__global__ void __launch_bounds__(UT) k_msb_update_r(MsState* st, MsBlockVecs v, long n,
-                                                     double* part) {
+SUSY_D void update_r_block(MsState* st, const MsBlockVecs& v, long n, double* part, int blk,
+                           int nblk) {
   static_assert(UT == ST, "the last block runs the ST-thread scalar step");
   static_assert(MS_MAXS <= ST, "one thread per shift");
   __shared__ double sh[ST / 32];
@@ -505,8 +542,7 @@ __global__ void __launch_bounds__(UT) k_msb_update_r(MsState* st, MsBlockVecs v,
   RT* rout = (RT*)v.ring[it % (MS_BLK + 1)];
   const MT* mp = (const MT*)(sizeof(MT) == 16 ? v.mp : v.mp32);
   double acc = 0.0;
-  // grid-stride: few blocks, so the scalar kernel sums few partials
-  for (long i = (long)blockIdx.x * UT + threadIdx.x; i < n; i += (long)gridDim.x * UT) {
+  for (long i = (long)blk * UT + threadIdx.x; i < n; i += (long)nblk * UT) {
     double2 r = ld2(rin, i);
     const MT m = mp[i];
     r.x += b0 * m.x;
@@ -517,21 +553,27 @@ __global__ void __launch_bounds__(UT) k_msb_update_r(MsState* st, MsBlockVecs v,
   }
   acc = block_sum<UT>(acc);
   if (threadIdx.x == 0) {
-    part[blockIdx.x] = acc;
+    part[blk] = acc;
     __threadfence();
-    last = atomicAdd(&st->done_r, 1u) == gridDim.x - 1;
+    last = atomicAdd(&st->done_r, 1u) == (unsigned)nblk - 1;
   }
   __syncthreads();
   if (!last) return;
   if (threadIdx.x == 0) st->done_r = 0;
-  scalars2_block(st, part, gridDim.x, sh);
+  scalars2_block(st, part, nblk, sh);
+}
+
+template <typename MT, typename RT>
+__global__ void __launch_bounds__(UT) k_msb_update_r(MsState* st, MsBlockVecs v, long n,
+                                                     double* part) {
+  update_r_block<MT, RT>(st, v, n, part, blockIdx.x, gridDim.x);
 }
 
 // p0 = r(i) + alpha_0 p0 (and its FP32 copy for an FP32 operator)
 template <typename RT>
-__global__ void __launch_bounds__(UT) k_msb_update_p0(MsState* st, MsBlockVecs v, long n) {
+SUSY_D void msb_p0_block(const MsState* st, const MsBlockVecs& v, long n, int blk) {
   if (st->skip_b) return;
-  const long i = (long)blockIdx.x * UT + threadIdx.x;
+  const long i = (long)blk * UT + threadIdx.x;
   if (i >= n) return;
   const double a0 = st->alpha[0];
   const double2 r = ld2((const RT*)v.ring[st->iter % (MS_BLK + 1)], i);
@@ -540,6 +582,11 @@ __global__ void __launch_bounds__(UT) k_msb_update_p0(MsState* st, MsBlockVecs v
   p.y = r.y + a0 * p.y;
   st2((RT*)v.p0, i, p);
   if (v.p0_32) ((float2*)v.p0_32)[i] = make_float2((float)p.x, (float)p.y);
+}
+
+template <typename RT>
+__global__ void __launch_bounds__(UT) k_msb_update_p0(MsState* st, MsBlockVecs v, long n) {
+  msb_p0_block<RT>(st, v, n, blockIdx.x);
 }
 
 // Residual replacement at a block boundary (k = st->iter): r(k) becomes the
@@ -598,55 +645,35 @@ __global__ void k_msb_set_rsq(MsState* st, double rsq) {
 }
 
 // The block pass: every live shift's psi_j and P_j advanced over the
-// recorded iterations.  Each CTA first derives the combination
-// coefficients of every live shift in shared memory.
+// recorded iterations, with the coefficients block_coefs left in the state
+// (blk: the block's index among the field's ceil(n / UT) blocks).
 template <typename RT>
-__global__ void __launch_bounds__(UT) k_msb_block(MsState* st, MsBlockVecs v, long n) {
+SUSY_D void block_pass(const MsState* st, const MsBlockVecs& v, long n, int blk) {
   __shared__ double cx0[MS_MAXS], cp0[MS_MAXS];
-  __shared__ double cxr[MS_MAXS][MS_BLK], cpr[MS_MAXS][MS_BLK];
+  __shared__ double cxr[MS_BLK][MS_MAXS], cpr[MS_BLK][MS_MAXS];
   __shared__ int lv[MS_MAXS];
   const int L = st->blk_len;
   if (L == 0) return;
   const int ns = st->nshift;
   const int k = st->blk_start;
-  if (threadIdx.x < ns) {
-    const int j = threadIdx.x;
-    lv[j] = st->live[j];
-    // c_t and d_{t,s} for t = 0..L, s = 1..t (d indexed s-1)
-    double c = 1.0, d[MS_BLK];
-    double x0 = 0.0, xr[MS_BLK];
-#pragma unroll
-    for (int q = 0; q < MS_BLK; q++) d[q] = xr[q] = 0.0;
-    for (int t = 0; t < L; t++) {
-      const double b = st->hb[t][j], z = st->hz[t][j], a = st->ha[t][j];
-      // psi -= b_t p(k + t)
-      x0 += b * c;
-#pragma unroll
-      for (int q = 0; q < MS_BLK; q++)
-        if (q < t) xr[q] += b * d[q];
-      // p(k + t + 1) = z_t R_{t+1} + a_t p(k + t)
-      c *= a;
-#pragma unroll
-      for (int q = 0; q < MS_BLK; q++) {
-        if (q < t) d[q] *= a;
-        if (q == t) d[q] = z;
-      }
-    }
-    cx0[j] = x0;
-    cp0[j] = c;
-#pragma unroll
-    for (int q = 0; q < MS_BLK; q++) {
-      cxr[j][q] = xr[q];
-      cpr[j][q] = d[q];
-    }
+  static_assert(MS_BLK * MS_MAXS <= UT, "one coefficient per thread");
+  if (threadIdx.x < MS_BLK * MS_MAXS) {
+    (&cxr[0][0])[threadIdx.x] = (&st->cxr[0][0])[threadIdx.x];
+    (&cpr[0][0])[threadIdx.x] = (&st->cpr[0][0])[threadIdx.x];
   }
-  __syncthreads();
-  const long i = (long)blockIdx.x * UT + threadIdx.x;
-  if (i >= n) return;
+  if (threadIdx.x < ns) {
+    lv[threadIdx.x] = st->live[threadIdx.x];
+    cx0[threadIdx.x] = st->cx0[threadIdx.x];
+    cp0[threadIdx.x] = st->cp0[threadIdx.x];
+  }
+  const long i = (long)blk * UT + threadIdx.x;
   double2 R[MS_BLK];
 #pragma unroll
   for (int q = 0; q < MS_BLK; q++)
-    R[q] = q < L ? ld2((const RT*)v.ring[(k + 1 + q) % (MS_BLK + 1)], i) : make_double2(0, 0);
+    R[q] = q < L && i < n ? ld2((const RT*)v.ring[(k + 1 + q) % (MS_BLK + 1)], i)
+                          : make_double2(0, 0);
+  __syncthreads();
+  if (i >= n) return;
 #pragma unroll 1
   for (int j = 0; j < ns; j++) {
     if (!lv[j]) continue;
@@ -661,18 +688,23 @@ __global__ void __launch_bounds__(UT) k_msb_block(MsState* st, MsBlockVecs v, lo
     pn.y = cp0[j] * p.y;
 #pragma unroll
     for (int q = 0; q < MS_BLK; q++) {
-      x.x -= cxr[j][q] * R[q].x;
-      x.y -= cxr[j][q] * R[q].y;
-      pn.x += cpr[j][q] * R[q].x;
-      pn.y += cpr[j][q] * R[q].y;
+      x.x -= cxr[q][j] * R[q].x;
+      x.y -= cxr[q][j] * R[q].y;
+      pn.x += cpr[q][j] * R[q].x;
+      pn.y += cpr[q][j] * R[q].y;
     }
     *xp = x;
     *pp = pn;
   }
 }
 
+template <typename RT>
+__global__ void __launch_bounds__(UT) k_msb_block(const MsState* st, MsBlockVecs v, long n) {
+  block_pass<RT>(st, v, n, blockIdx.x);
+}
+
 // Close the block: shifts frozen by now take no part in later blocks
-__global__ void k_msb_block_reset(MsState* st) {
+SUSY_D void block_reset(MsState* st) {
   const int j = threadIdx.x;
   if (j < MS_MAXS) st->live[j] = j < st->nshift && (j == 0 || !st->converged[j]);
   __syncthreads();
@@ -681,6 +713,7 @@ __global__ void k_msb_block_reset(MsState* st) {
     st->blk_len = 0;
   }
 }
+__global__ void k_msb_block_reset(MsState* st) { block_reset(st); }
 
 // Returns the number of partials written (at most 8 blocks per SM of a
 // 148-SM B200)
@@ -754,20 +787,24 @@ void norm2_partials(const void* x, int prec, long n, double* part, cudaStream_t 
 }  // namespace susy
 
 // ---------------------------------------------------------------------------
-// Batched FP64 multi-shift solve: the per-iteration kernels above for every
+// Batched FP64 multi-shift solve: the kernels of the blocked solver for every
 // lattice of a batch in one launch each.  The recurrence kernels run one
 // block per lattice; the vector kernels walk a table of vector blocks in
-// which lattice i owns blocks [vblk0, vblk0 + vblocks).  Each lattice's
-// state, stop flag and partials are its own, so every lattice follows the
-// solo recurrences and stops at its own iteration.
+// which lattice i owns blocks [rblk0, rblk0 + rblocks) of the residual update
+// (its last block runs the lattice's second recurrences) and
+// [vblk0, vblk0 + vblocks) of the others.  Each lattice's state, stop flag
+// and partials are its own, so every lattice follows the solo recurrences
+// and stops at its own iteration.
 namespace susy {
 
-// Largest i < nl with L[i].vblk0 <= b
+// Largest i < nl whose first block of the table (RT: the residual update's)
+// is <= b
+template <bool RT>
 SUSY_D int vblock_lattice(const MsLat* L, int nl, int b) {
   int lo = 0, hi = nl - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    if (L[mid].vblk0 <= b)
+    if ((RT ? L[mid].rblk0 : L[mid].vblk0) <= b)
       lo = mid;
     else
       hi = mid - 1;
@@ -781,39 +818,43 @@ __global__ void k_msbat_scalars1(const MsLat* L) {
   scalars1_block(l.st, l.part0, l.np0, sh);
 }
 
-__global__ void k_msbat_scalars2(const MsLat* L) {
-  __shared__ double sh[ST / 32];
-  const MsLat& l = L[blockIdx.x];
-  if (l.st->skip) return;
-  scalars2_block(l.st, l.part1, l.vblocks, sh);
-}
-
-__global__ void __launch_bounds__(UT) k_msbat_update_fused(const MsLat* L, int nl) {
-  const MsLat& l = L[vblock_lattice(L, nl, blockIdx.x)];
-  update_fused_block<double2, double2>(l.st, l.v, l.n, l.part1, blockIdx.x - l.vblk0);
+__global__ void __launch_bounds__(UT) k_msbat_update_r(const MsLat* L, int nl) {
+  const MsLat& l = L[vblock_lattice<true>(L, nl, blockIdx.x)];
+  update_r_block<double2, double2>(l.st, l.v, l.n, l.part1, blockIdx.x - l.rblk0, l.rblocks);
 }
 
 __global__ void __launch_bounds__(UT) k_msbat_update_p0(const MsLat* L, int nl) {
-  const MsLat& l = L[vblock_lattice(L, nl, blockIdx.x)];
-  update_p0_block<double2>(l.st, l.v, l.n, blockIdx.x - l.vblk0);
+  const MsLat& l = L[vblock_lattice<false>(L, nl, blockIdx.x)];
+  msb_p0_block<double2>(l.st, l.v, l.n, blockIdx.x - l.vblk0);
 }
+
+__global__ void __launch_bounds__(UT) k_msbat_block(const MsLat* L, int nl) {
+  const MsLat& l = L[vblock_lattice<false>(L, nl, blockIdx.x)];
+  block_pass<double2>(l.st, l.v, l.n, blockIdx.x - l.vblk0);
+}
+
+__global__ void k_msbat_block_reset(const MsLat* L) { block_reset(L[blockIdx.x].st); }
 
 __global__ void k_msbat_skips(const MsLat* L, int nl, int* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < nl) out[i] = L[i].st->skip;
 }
 
+// Four elements a thread in the residual update of a lattice of n elements
+int msbat_rblocks(long n) { return (int)((n + 4 * UT - 1) / (4 * UT)); }
+
 void ms_batch_scalars1(const MsLat* L, int nl, cudaStream_t s) {
   count_launch(), k_msbat_scalars1<<<nl, ST, 0, s>>>(L);
 }
-void ms_batch_update_fused(const MsLat* L, int nl, int vtot, cudaStream_t s) {
-  count_launch(), k_msbat_update_fused<<<vtot, UT, 0, s>>>(L, nl);
-}
-void ms_batch_scalars2(const MsLat* L, int nl, cudaStream_t s) {
-  count_launch(), k_msbat_scalars2<<<nl, ST, 0, s>>>(L);
+void ms_batch_update_r(const MsLat* L, int nl, int rtot, cudaStream_t s) {
+  count_launch(), k_msbat_update_r<<<rtot, UT, 0, s>>>(L, nl);
 }
 void ms_batch_update_p0(const MsLat* L, int nl, int vtot, cudaStream_t s) {
   count_launch(), k_msbat_update_p0<<<vtot, UT, 0, s>>>(L, nl);
+}
+void ms_batch_block(const MsLat* L, int nl, int vtot, cudaStream_t s) {
+  count_launch(), k_msbat_block<<<vtot, UT, 0, s>>>(L, nl);
+  count_launch(), k_msbat_block_reset<<<nl, MS_MAXS, 0, s>>>(L);
 }
 void ms_batch_skips(const MsLat* L, int nl, int* out, cudaStream_t s) {
   count_launch(), k_msbat_skips<<<(nl + 63) / 64, 64, 0, s>>>(L, nl, out);

@@ -33,6 +33,8 @@ struct MsState {
   unsigned done_r;    // blocks of the fused residual update finished so far
   int live[MS_MAXS];
   double hb[MS_BLK][MS_MAXS], hz[MS_BLK][MS_MAXS], ha[MS_BLK][MS_MAXS];
+  // the block's combination coefficients (block_coefs, cg.cu)
+  double cx0[MS_MAXS], cp0[MS_MAXS], cxr[MS_BLK][MS_MAXS], cpr[MS_BLK][MS_MAXS];
   double shift[MS_MAXS];
   double zeta_i[MS_MAXS], zeta_im1[MS_MAXS], zeta_ip1[MS_MAXS];
   double beta_i[MS_MAXS], beta_im1[MS_MAXS], alpha[MS_MAXS];
@@ -180,24 +182,25 @@ void msb_block(MsState* st, const MsBlockVecs& v, long n, cudaStream_t s);
 void ms_set_stop(MsState* st, double errormin_base, cudaStream_t s);
 
 // One lattice of a batched FP64 multi-shift solve (solver.cu): its state,
-// vectors, field size, the operator's dot partials and the vector update's
-// |r|^2 partials, and its blocks in the batch's table of vector blocks.
+// vectors, field size, the operator's dot partials and the residual update's
+// |r|^2 partials, and its blocks in the batch's tables of vector blocks.
 struct MsLat {
   MsState* st;
-  MsVecs v;
+  MsBlockVecs v;
   long n;          // complex entries of one Twist_Fermion
   double* part0;   // operator partials (16 ceil(V / 128) of them)
   int np0;
-  double* part1;   // |r|^2 partials, one per vector block
-  int vblk0;       // the lattice's first block in the batch's vector table
-  int vblocks;     // its vector blocks, vec_blocks(n)
+  double* part1;   // |r|^2 partials, one per block of the residual update
+  int rblk0, rblocks;   // first block and blocks in the residual update's table
+  int vblk0, vblocks;   // and in the other vector kernels' (vec_blocks(n))
 };
-// The per-iteration kernels of ms_run for every lattice of a batch at once
-// (L: a device array of nl MsLat; vtot: vector blocks of all lattices)
+int msbat_rblocks(long n);
+// The kernels of the blocked solver for every lattice of a batch at once
+// (L: a device array of nl MsLat; rtot, vtot: table sizes)
 void ms_batch_scalars1(const MsLat* L, int nl, cudaStream_t s);
-void ms_batch_update_fused(const MsLat* L, int nl, int vtot, cudaStream_t s);
-void ms_batch_scalars2(const MsLat* L, int nl, cudaStream_t s);
+void ms_batch_update_r(const MsLat* L, int nl, int rtot, cudaStream_t s);
 void ms_batch_update_p0(const MsLat* L, int nl, int vtot, cudaStream_t s);
+void ms_batch_block(const MsLat* L, int nl, int vtot, cudaStream_t s);
 // out[i] = lattice i's stop flag
 void ms_batch_skips(const MsLat* L, int nl, int* out, cudaStream_t s);
 
