@@ -124,6 +124,7 @@ SUSY_D void scalars1_block(MsState* st, const double* partials, int np, double* 
 
 __global__ void k_ms_scalars1(MsState* st, const double* partials, int np) {
   __shared__ double sh[ST / 32];
+  wait_prior();
   scalars1_block(st, partials, np, sh);
 }
 
@@ -393,7 +394,7 @@ void ms_init(MsState* st, const void* src, int prec, long n, double* part, int m
 }
 
 void ms_scalars1(MsState* st, const double* part, int np, cudaStream_t s) {
-  count_launch(), k_ms_scalars1<<<1, ST, 0, s>>>(st, part, np);
+  launch_dep(k_ms_scalars1, 1, ST, s, st, part, np);
 }
 
 void ms_scalars2(MsState* st, const double* part, int np, cudaStream_t s) {
@@ -566,6 +567,7 @@ SUSY_D void update_r_block(MsState* st, const MsBlockVecs& v, long n, double* pa
 template <typename MT, typename RT>
 __global__ void __launch_bounds__(UT) k_msb_update_r(MsState* st, MsBlockVecs v, long n,
                                                      double* part) {
+  wait_prior();
   update_r_block<MT, RT>(st, v, n, part, blockIdx.x, gridDim.x);
 }
 
@@ -586,6 +588,7 @@ SUSY_D void msb_p0_block(const MsState* st, const MsBlockVecs& v, long n, int bl
 
 template <typename RT>
 __global__ void __launch_bounds__(UT) k_msb_update_p0(MsState* st, MsBlockVecs v, long n) {
+  wait_prior();
   msb_p0_block<RT>(st, v, n, blockIdx.x);
 }
 
@@ -700,6 +703,7 @@ SUSY_D void block_pass(const MsState* st, const MsBlockVecs& v, long n, int blk)
 
 template <typename RT>
 __global__ void __launch_bounds__(UT) k_msb_block(const MsState* st, MsBlockVecs v, long n) {
+  wait_prior();
   block_pass<RT>(st, v, n, blockIdx.x);
 }
 
@@ -713,7 +717,10 @@ SUSY_D void block_reset(MsState* st) {
     st->blk_len = 0;
   }
 }
-__global__ void k_msb_block_reset(MsState* st) { block_reset(st); }
+__global__ void k_msb_block_reset(MsState* st) {
+  wait_prior();
+  block_reset(st);
+}
 
 // Returns the number of partials written (at most 8 blocks per SM of a
 // 148-SM B200)
@@ -721,11 +728,11 @@ void msb_update_r(MsState* st, const MsBlockVecs& v, long n, double* part, bool 
                   cudaStream_t s) {
   const int nb = vec_blocks(n) < 1184 ? vec_blocks(n) : 1184;
   if (v.f32)
-    count_launch(), k_msb_update_r<float2, float2><<<nb, UT, 0, s>>>(st, v, n, part);
+    launch_dep(k_msb_update_r<float2, float2>, nb, UT, s, st, v, n, part);
   else if (mp32)
-    count_launch(), k_msb_update_r<float2, double2><<<nb, UT, 0, s>>>(st, v, n, part);
+    launch_dep(k_msb_update_r<float2, double2>, nb, UT, s, st, v, n, part);
   else
-    count_launch(), k_msb_update_r<double2, double2><<<nb, UT, 0, s>>>(st, v, n, part);
+    launch_dep(k_msb_update_r<double2, double2>, nb, UT, s, st, v, n, part);
 }
 
 // Residual replacement: r(k) <- rt with the matching search-vector
@@ -742,17 +749,17 @@ void msb_replace(MsState* st, const MsBlockVecs& v, long n, const void* rt, doub
 
 void msb_update_p0(MsState* st, const MsBlockVecs& v, long n, cudaStream_t s) {
   if (v.f32)
-    count_launch(), k_msb_update_p0<float2><<<vec_blocks(n), UT, 0, s>>>(st, v, n);
+    launch_dep(k_msb_update_p0<float2>, vec_blocks(n), UT, s, st, v, n);
   else
-    count_launch(), k_msb_update_p0<double2><<<vec_blocks(n), UT, 0, s>>>(st, v, n);
+    launch_dep(k_msb_update_p0<double2>, vec_blocks(n), UT, s, st, v, n);
 }
 
 void msb_block(MsState* st, const MsBlockVecs& v, long n, cudaStream_t s) {
   if (v.f32)
-    count_launch(), k_msb_block<float2><<<vec_blocks(n), UT, 0, s>>>(st, v, n);
+    launch_dep(k_msb_block<float2>, vec_blocks(n), UT, s, st, v, n);
   else
-    count_launch(), k_msb_block<double2><<<vec_blocks(n), UT, 0, s>>>(st, v, n);
-  count_launch(), k_msb_block_reset<<<1, MS_MAXS, 0, s>>>(st);
+    launch_dep(k_msb_block<double2>, vec_blocks(n), UT, s, st, v, n);
+  launch_dep(k_msb_block_reset, 1, MS_MAXS, s, st);
 }
 
 // Re <a, b> partials over n FP64 complex entries
@@ -814,26 +821,33 @@ SUSY_D int vblock_lattice(const MsLat* L, int nl, int b) {
 
 __global__ void k_msbat_scalars1(const MsLat* L) {
   __shared__ double sh[ST / 32];
+  wait_prior();
   const MsLat& l = L[blockIdx.x];
   scalars1_block(l.st, l.part0, l.np0, sh);
 }
 
 __global__ void __launch_bounds__(UT) k_msbat_update_r(const MsLat* L, int nl) {
+  wait_prior();
   const MsLat& l = L[vblock_lattice<true>(L, nl, blockIdx.x)];
   update_r_block<double2, double2>(l.st, l.v, l.n, l.part1, blockIdx.x - l.rblk0, l.rblocks);
 }
 
 __global__ void __launch_bounds__(UT) k_msbat_update_p0(const MsLat* L, int nl) {
+  wait_prior();
   const MsLat& l = L[vblock_lattice<false>(L, nl, blockIdx.x)];
   msb_p0_block<double2>(l.st, l.v, l.n, blockIdx.x - l.vblk0);
 }
 
 __global__ void __launch_bounds__(UT) k_msbat_block(const MsLat* L, int nl) {
+  wait_prior();
   const MsLat& l = L[vblock_lattice<false>(L, nl, blockIdx.x)];
   block_pass<double2>(l.st, l.v, l.n, blockIdx.x - l.vblk0);
 }
 
-__global__ void k_msbat_block_reset(const MsLat* L) { block_reset(L[blockIdx.x].st); }
+__global__ void k_msbat_block_reset(const MsLat* L) {
+  wait_prior();
+  block_reset(L[blockIdx.x].st);
+}
 
 __global__ void k_msbat_skips(const MsLat* L, int nl, int* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -844,17 +858,17 @@ __global__ void k_msbat_skips(const MsLat* L, int nl, int* out) {
 int msbat_rblocks(long n) { return (int)((n + 4 * UT - 1) / (4 * UT)); }
 
 void ms_batch_scalars1(const MsLat* L, int nl, cudaStream_t s) {
-  count_launch(), k_msbat_scalars1<<<nl, ST, 0, s>>>(L);
+  launch_dep(k_msbat_scalars1, nl, ST, s, L);
 }
 void ms_batch_update_r(const MsLat* L, int nl, int rtot, cudaStream_t s) {
-  count_launch(), k_msbat_update_r<<<rtot, UT, 0, s>>>(L, nl);
+  launch_dep(k_msbat_update_r, rtot, UT, s, L, nl);
 }
 void ms_batch_update_p0(const MsLat* L, int nl, int vtot, cudaStream_t s) {
-  count_launch(), k_msbat_update_p0<<<vtot, UT, 0, s>>>(L, nl);
+  launch_dep(k_msbat_update_p0, vtot, UT, s, L, nl);
 }
 void ms_batch_block(const MsLat* L, int nl, int vtot, cudaStream_t s) {
-  count_launch(), k_msbat_block<<<vtot, UT, 0, s>>>(L, nl);
-  count_launch(), k_msbat_block_reset<<<nl, MS_MAXS, 0, s>>>(L);
+  launch_dep(k_msbat_block, vtot, UT, s, L, nl);
+  launch_dep(k_msbat_block_reset, nl, MS_MAXS, s, L);
 }
 void ms_batch_skips(const MsLat* L, int nl, int* out, cudaStream_t s) {
   count_launch(), k_msbat_skips<<<(nl + 63) / 64, 64, 0, s>>>(L, nl, out);

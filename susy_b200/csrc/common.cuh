@@ -301,3 +301,32 @@ SUSY_D double block_sum(double v) {
   return r;
 }
 }  // namespace susy
+
+namespace susy {
+// Programmatic dependent launch: a kernel launched with launch_dep may be
+// scheduled while the kernel before it in the stream drains, so the launch
+// latency and the ramp of its blocks overlap that tail.  Its threads call
+// wait_prior() before they touch anything an earlier kernel wrote (or that
+// one may still read); it returns once that kernel, which did the same, is
+// complete and its writes are visible, so the order of the stream holds
+// throughout.  Every kernel launched this way calls it on every path.
+SUSY_D void wait_prior() {
+  cudaGridDependencySynchronize();
+  cudaTriggerProgrammaticLaunchCompletion();
+}
+
+template <typename... P, typename... A>
+inline void launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+  cudaLaunchAttribute at;
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = st;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  count_launch();
+  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+}  // namespace susy

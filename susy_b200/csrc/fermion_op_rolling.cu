@@ -290,6 +290,7 @@ SUSY_D double rl_site(const FopArgs<R>& a, int comp, int s0) {
 
 template <int N, typename R, int SIGN, int MINB>
 __global__ void __launch_bounds__(RL_THREADS, MINB) fermion_op_rolling_kernel(FopArgs<R> a) {
+  wait_prior();
   if (a.skip && *a.skip) return;
   double part = rl_site<N, R, SIGN>(a, blockIdx.x % NTF,
                                     (blockIdx.x / NTF) * RL_THREADS + threadIdx.x);
@@ -304,11 +305,11 @@ static int launch_rolling(FopArgs<R> a, int sign, cudaStream_t st) {
   const int nb = (a.g.V + RL_THREADS - 1) / RL_THREADS;
   const dim3 nt(nb, NUMLINK + 1);
   if (sign > 0) {
-    if (a.doG && !a.traces_ready) count_launch(), k_det_traces<N, R, false><<<nt, RL_THREADS, 0, st>>>(a);
-    count_launch(), fermion_op_rolling_kernel<N, R, 1, MINB><<<nb * NTF, RL_THREADS, 0, st>>>(a);
+    if (a.doG && !a.traces_ready) launch_dep(k_det_traces<N, R, false>, nt, RL_THREADS, st, a);
+    launch_dep(fermion_op_rolling_kernel<N, R, 1, MINB>, nb * NTF, RL_THREADS, st, a);
   } else {
-    if (a.doG && !a.traces_ready) count_launch(), k_det_traces<N, R, true><<<nt, RL_THREADS, 0, st>>>(a);
-    count_launch(), fermion_op_rolling_kernel<N, R, -1, MINB><<<nb * NTF, RL_THREADS, 0, st>>>(a);
+    if (a.doG && !a.traces_ready) launch_dep(k_det_traces<N, R, true>, nt, RL_THREADS, st, a);
+    launch_dep(fermion_op_rolling_kernel<N, R, -1, MINB>, nb * NTF, RL_THREADS, st, a);
   }
   return nb * NTF;
 }
@@ -371,6 +372,7 @@ SUSY_D int batch_lattice(const int* start, int n, int t) {
 template <int N, typename R, int SIGN, int MINB>
 __global__ void __launch_bounds__(RL_THREADS, MINB)
 fermion_op_batch_kernel(const __grid_constant__ FopBatch<R> B) {
+  wait_prior();
   const int total = NTF * B.tiles;
 #pragma unroll 1
   for (int w = blockIdx.x; w < total; w += gridDim.x) {
@@ -391,6 +393,7 @@ fermion_op_batch_kernel(const __grid_constant__ FopBatch<R> B) {
 // The trace pre-pass of every lattice: block (gt, e)
 template <int N, typename R, bool ADJ>
 __global__ void k_det_traces_batch(const __grid_constant__ FopBatch<R> B) {
+  wait_prior();
   const int i = batch_lattice(B.start, B.n, blockIdx.x);
   const FopArgs<R>& a = B.a[i];
   if (!a.doG || (a.skip && *a.skip)) return;
@@ -402,11 +405,11 @@ static void launch_batch(const FopBatch<R>& B, int sign, bool traces, int sms, c
   const int grid = NTF * B.tiles < MINB * sms ? NTF * B.tiles : MINB * sms;
   const dim3 nt(B.tiles, NUMLINK + 1);
   if (sign > 0) {
-    if (traces) count_launch(), k_det_traces_batch<N, R, false><<<nt, RL_THREADS, 0, st>>>(B);
-    count_launch(), fermion_op_batch_kernel<N, R, 1, MINB><<<grid, RL_THREADS, 0, st>>>(B);
+    if (traces) launch_dep(k_det_traces_batch<N, R, false>, nt, RL_THREADS, st, B);
+    launch_dep(fermion_op_batch_kernel<N, R, 1, MINB>, grid, RL_THREADS, st, B);
   } else {
-    if (traces) count_launch(), k_det_traces_batch<N, R, true><<<nt, RL_THREADS, 0, st>>>(B);
-    count_launch(), fermion_op_batch_kernel<N, R, -1, MINB><<<grid, RL_THREADS, 0, st>>>(B);
+    if (traces) launch_dep(k_det_traces_batch<N, R, true>, nt, RL_THREADS, st, B);
+    launch_dep(fermion_op_batch_kernel<N, R, -1, MINB>, grid, RL_THREADS, st, B);
   }
 }
 

@@ -248,6 +248,7 @@ SUSY_D void det_traces_site(const FopArgs<R>& a, int s, int e) {
 }
 template <int N, typename R, bool ADJ>
 __global__ void k_det_traces(FopArgs<R> a) {
+  wait_prior();
   if (a.skip && *a.skip) return;
   det_traces_site<N, R, ADJ>(a, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y);
 }
