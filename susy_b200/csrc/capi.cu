@@ -182,6 +182,13 @@ int dev_fop(susy_b200_lattice* h, const void* src, void* dst, int sign, int prec
   return launch_variant(h, src, dst, sign, prec, add, addc, dot, skip, h->fop_variant[pi], chain);
 }
 
+bool fop_uses_traces(susy_b200_lattice* h, int prec) {
+  const int pi = prec == 64 ? 0 : 1;
+  if (h->fop_variant[pi] < 0) autotune_fop(h, prec);
+  return h->trace[pi] &&
+         (h->fop_variant[pi] == FOP_ROLLING || h->fop_variant[pi] == FOP_ROLLING_WIDE);
+}
+
 void* scratch_tf(susy_b200_lattice* h, int which, int prec) {
   void** slot = prec == 64 ? &h->tf64[which] : &h->tf32[which];
   if (!*slot) *slot = dalloc(h, field_bytes(h, NTF, prec));
@@ -257,6 +264,7 @@ susy_b200_lattice* solver_shadow(susy_b200_lattice* h) {
   c->G = h->G;
   c->ms_blocked = h->ms_blocked;
   c->use_graphs = h->use_graphs;
+  c->graphs_asked = h->graphs_asked;
   c->mix_switch = h->mix_switch;
   c->mix_reliable = h->mix_reliable;
   c->mix_interval = h->mix_interval;
@@ -449,7 +457,7 @@ int susy_b200_set_solver(susy_b200_lattice* h, int solver) {
 int susy_b200_use_graphs(susy_b200_lattice* h, int on) {
   if (!h) return SUSY_B200_EINVAL;
   const int prev = h->use_graphs;
-  if (on >= 0) h->use_graphs = on ? 1 : 0;
+  if (on >= 0) h->use_graphs = h->graphs_asked = on ? 1 : 0;
   return prev;
 }
 

@@ -565,32 +565,65 @@ SUSY_D void update_r_block(MsState* st, const MsBlockVecs& v, long n, double* pa
 }
 
 template <typename MT, typename RT>
-__global__ void __launch_bounds__(UT) k_msb_update_r(MsState* st, MsBlockVecs v, long n,
-                                                     double* part) {
+// six blocks per SM: the coefficient step of the last block must not cost the
+// streaming loop its occupancy (58 us a launch at 12^3x24 U(3) with four, 51
+// with six)
+__global__ void __launch_bounds__(UT, 6) k_msb_update_r(MsState* st, MsBlockVecs v, long n,
+                                                        double* part) {
   wait_prior();
   update_r_block<MT, RT>(st, v, n, part, blockIdx.x, gridDim.x);
 }
 
-// p0 = r(i) + alpha_0 p0 (and its FP32 copy for an FP32 operator)
-template <typename RT>
-SUSY_D void msb_p0_block(const MsState* st, const MsBlockVecs& v, long n, int blk) {
+// p0 = r(i) + alpha_0 p0 (and its FP32 copy for an FP32 operator), and with a
+// trace field the traces of the operator's input (k_det_traces, summed in the
+// same order), which saves the next D its pre-pass and a read of the link
+// components.  Block (tile, k) holds component k of 256 sites, a thread the
+// N^2 elements of one site.  OR: the operator's precision.  8^4 U(2) solve
+// 7.50 -> 7.03 ms with it.  (The residual update in the same layout took 71
+// against 58 us at 12^3x24 U(3): it stays element-linear.)
+template <int N, typename RT, typename OR>
+SUSY_D void msb_p0_block(const MsState* st, const MsBlockVecs& v, int blk) {
   if (st->skip_b) return;
-  const long i = (long)blk * UT + threadIdx.x;
-  if (i >= n) return;
+  const int k = blk % NTF, s = (blk / NTF) * UT + threadIdx.x;
+  if (s >= v.S) return;
+  const long o = (long)(k * N * N) * v.S + s;
   const double a0 = st->alpha[0];
-  const double2 r = ld2((const RT*)v.ring[st->iter % (MS_BLK + 1)], i);
-  double2 p = ld2((const RT*)v.p0, i);
-  p.x = r.x + a0 * p.x;
-  p.y = r.y + a0 * p.y;
-  st2((RT*)v.p0, i, p);
-  if (v.p0_32) ((float2*)v.p0_32)[i] = make_float2((float)p.x, (float)p.y);
+  const RT* rp = (const RT*)v.ring[st->iter % (MS_BLK + 1)] + o;
+  RT* pp = (RT*)v.p0 + o;
+  Mat<N, OR> m;
+#pragma unroll
+  for (int e = 0; e < N * N; e++) {
+    const double2 r = ld2(rp, (long)e * v.S);
+    double2 p = ld2((const RT*)pp, (long)e * v.S);
+    p.x = r.x + a0 * p.x;
+    p.y = r.y + a0 * p.y;
+    st2(pp, (long)e * v.S, p);
+    if (v.p0_32) ((float2*)v.p0_32)[o + (long)e * v.S] = make_float2((float)p.x, (float)p.y);
+    m.e[e / N][e % N] = Cx<OR>((OR)p.x, (OR)p.y);
+  }
+  if (!v.trace || k > NUMLINK) return;
+  typedef typename CT<OR>::T T;
+  Cx<OR> t(0, 0);
+  if (k == 0) {
+#pragma unroll
+    for (int i = 0; i < N; i++) t = t + m.e[i][i];
+  } else {
+    const T* pu = (const T*)v.Uinv + (long)((k - 1) * N * N) * v.S + s;
+#pragma unroll
+    for (int i = 0; i < N; i++)
+#pragma unroll
+      for (int j = 0; j < N; j++) t = t + ldc<OR>(pu + (long)(i * N + j) * v.S) * m.e[j][i];
+  }
+  stc<OR>((T*)v.trace + (long)(k == 0 ? NUMLINK : k - 1) * v.S + s, t);
 }
 
-template <typename RT>
-__global__ void __launch_bounds__(UT) k_msb_update_p0(MsState* st, MsBlockVecs v, long n) {
+template <int N, typename RT, typename OR>
+__global__ void __launch_bounds__(UT) k_msb_update_p0(MsState* st, MsBlockVecs v) {
   wait_prior();
-  msb_p0_block<RT>(st, v, n, blockIdx.x);
+  msb_p0_block<N, RT, OR>(st, v, blockIdx.x);
 }
+
+int msb_p0_blocks(int S) { return NTF * ((S + UT - 1) / UT); }
 
 // Residual replacement at a block boundary (k = st->iter): r(k) becomes the
 // true residual rt, and the search vectors built from the old r(k) get the
@@ -722,11 +755,12 @@ __global__ void k_msb_block_reset(MsState* st) {
   block_reset(st);
 }
 
-// Returns the number of partials written (at most 8 blocks per SM of a
-// 148-SM B200)
+// Four elements a thread, at most the 6 blocks per SM of a 148-SM B200 that
+// are resident: each block costs a fenced partial and an atomic, and the last
+// one sums them all (at 8^4 U(2) 256 blocks in place of 1024)
 void msb_update_r(MsState* st, const MsBlockVecs& v, long n, double* part, bool mp32,
                   cudaStream_t s) {
-  const int nb = vec_blocks(n) < 1184 ? vec_blocks(n) : 1184;
+  const int nb = msbat_rblocks(n) < 888 ? msbat_rblocks(n) : 888;
   if (v.f32)
     launch_dep(k_msb_update_r<float2, float2>, nb, UT, s, st, v, n, part);
   else if (mp32)
@@ -747,11 +781,23 @@ void msb_replace(MsState* st, const MsBlockVecs& v, long n, const void* rt, doub
   count_launch(), k_msb_set_rsq<<<1, 1, 0, s>>>(st, rsq);
 }
 
-void msb_update_p0(MsState* st, const MsBlockVecs& v, long n, cudaStream_t s) {
+template <int N>
+static void launch_update_p0(MsState* st, const MsBlockVecs& v, cudaStream_t s) {
+  const int nb = msb_p0_blocks(v.S);
   if (v.f32)
-    launch_dep(k_msb_update_p0<float2>, vec_blocks(n), UT, s, st, v, n);
+    launch_dep(k_msb_update_p0<N, float2, float>, nb, UT, s, st, v);
+  else if (v.p0_32)
+    launch_dep(k_msb_update_p0<N, double2, float>, nb, UT, s, st, v);
   else
-    launch_dep(k_msb_update_p0<double2>, vec_blocks(n), UT, s, st, v, n);
+    launch_dep(k_msb_update_p0<N, double2, double>, nb, UT, s, st, v);
+}
+
+void msb_update_p0(MsState* st, const MsBlockVecs& v, cudaStream_t s) {
+  switch (v.N) {
+    case 2: launch_update_p0<2>(st, v, s); break;
+    case 3: launch_update_p0<3>(st, v, s); break;
+    default: launch_update_p0<4>(st, v, s); break;
+  }
 }
 
 void msb_block(MsState* st, const MsBlockVecs& v, long n, cudaStream_t s) {
@@ -798,20 +844,19 @@ void norm2_partials(const void* x, int prec, long n, double* part, cudaStream_t 
 // lattice of a batch in one launch each.  The recurrence kernels run one
 // block per lattice; the vector kernels walk a table of vector blocks in
 // which lattice i owns blocks [rblk0, rblk0 + rblocks) of the residual update
-// (its last block runs the lattice's second recurrences) and
-// [vblk0, vblk0 + vblocks) of the others.  Each lattice's state, stop flag
+// (its last block runs the lattice's second recurrences), [qblk0, ...) of the
+// p0 update and [vblk0, ...) of the block pass.  Each lattice's state, stop flag
 // and partials are its own, so every lattice follows the solo recurrences
 // and stops at its own iteration.
 namespace susy {
 
-// Largest i < nl whose first block of the table (RT: the residual update's)
-// is <= b
-template <bool RT>
+// Largest i < nl whose first block in table T is <= b
+template <int MsLat::* T>
 SUSY_D int vblock_lattice(const MsLat* L, int nl, int b) {
   int lo = 0, hi = nl - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    if ((RT ? L[mid].rblk0 : L[mid].vblk0) <= b)
+    if (L[mid].*T <= b)
       lo = mid;
     else
       hi = mid - 1;
@@ -826,21 +871,22 @@ __global__ void k_msbat_scalars1(const MsLat* L) {
   scalars1_block(l.st, l.part0, l.np0, sh);
 }
 
-__global__ void __launch_bounds__(UT) k_msbat_update_r(const MsLat* L, int nl) {
+__global__ void __launch_bounds__(UT, 6) k_msbat_update_r(const MsLat* L, int nl) {
   wait_prior();
-  const MsLat& l = L[vblock_lattice<true>(L, nl, blockIdx.x)];
+  const MsLat& l = L[vblock_lattice<&MsLat::rblk0>(L, nl, blockIdx.x)];
   update_r_block<double2, double2>(l.st, l.v, l.n, l.part1, blockIdx.x - l.rblk0, l.rblocks);
 }
 
+template <int N>
 __global__ void __launch_bounds__(UT) k_msbat_update_p0(const MsLat* L, int nl) {
   wait_prior();
-  const MsLat& l = L[vblock_lattice<false>(L, nl, blockIdx.x)];
-  msb_p0_block<double2>(l.st, l.v, l.n, blockIdx.x - l.vblk0);
+  const MsLat& l = L[vblock_lattice<&MsLat::qblk0>(L, nl, blockIdx.x)];
+  msb_p0_block<N, double2, double>(l.st, l.v, blockIdx.x - l.qblk0);
 }
 
 __global__ void __launch_bounds__(UT) k_msbat_block(const MsLat* L, int nl) {
   wait_prior();
-  const MsLat& l = L[vblock_lattice<false>(L, nl, blockIdx.x)];
+  const MsLat& l = L[vblock_lattice<&MsLat::vblk0>(L, nl, blockIdx.x)];
   block_pass<double2>(l.st, l.v, l.n, blockIdx.x - l.vblk0);
 }
 
@@ -854,7 +900,6 @@ __global__ void k_msbat_skips(const MsLat* L, int nl, int* out) {
   if (i < nl) out[i] = L[i].st->skip;
 }
 
-// Four elements a thread in the residual update of a lattice of n elements
 int msbat_rblocks(long n) { return (int)((n + 4 * UT - 1) / (4 * UT)); }
 
 void ms_batch_scalars1(const MsLat* L, int nl, cudaStream_t s) {
@@ -863,8 +908,12 @@ void ms_batch_scalars1(const MsLat* L, int nl, cudaStream_t s) {
 void ms_batch_update_r(const MsLat* L, int nl, int rtot, cudaStream_t s) {
   launch_dep(k_msbat_update_r, rtot, UT, s, L, nl);
 }
-void ms_batch_update_p0(const MsLat* L, int nl, int vtot, cudaStream_t s) {
-  launch_dep(k_msbat_update_p0, vtot, UT, s, L, nl);
+void ms_batch_update_p0(const MsLat* L, int nl, int N, int qtot, cudaStream_t s) {
+  switch (N) {
+    case 2: launch_dep(k_msbat_update_p0<2>, qtot, UT, s, L, nl); break;
+    case 3: launch_dep(k_msbat_update_p0<3>, qtot, UT, s, L, nl); break;
+    default: launch_dep(k_msbat_update_p0<4>, qtot, UT, s, L, nl); break;
+  }
 }
 void ms_batch_block(const MsLat* L, int nl, int vtot, cudaStream_t s) {
   launch_dep(k_msbat_block, vtot, UT, s, L, nl);

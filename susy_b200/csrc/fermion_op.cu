@@ -283,10 +283,11 @@ int fermion_op(const Geo& g, int N, const void* U, const void* Uinv, const void*
   if (variant == FOP_ROWS) return fermion_op_rows<R>(a, N, sign, st);
   const bool rolling = variant == FOP_ROLLING || variant == FOP_ROLLING_WIDE;
   if (rolling && !trace) variant = FOP_SITE_MAJOR_FRONT;
-  if (rolling && trace && a.doG && chain == FOP_FIRST) a.trace_out = (T*)trace + 6 * (size_t)g.S;
-  if (rolling && trace && a.doG && chain == FOP_SECOND) {
-    a.trace = (T*)trace + 6 * (size_t)g.S;
-    a.traces_ready = 1;
+  if (rolling && trace && a.doG) {
+    T* second = (T*)trace + 6 * (size_t)g.S;
+    if (chain == FOP_FIRST || chain == FOP_TRACED) a.trace_out = second;
+    if (chain == FOP_SECOND) a.trace = second;
+    a.traces_ready = chain == FOP_SECOND || chain == FOP_TRACED;
   }
   if (rolling && trace) return fermion_op_rolling<R>(a, N, sign, variant == FOP_ROLLING_WIDE, st);
   if (variant >= FOP_COMPACT) return fermion_op_compact<R>(a, N, sign, variant, st);

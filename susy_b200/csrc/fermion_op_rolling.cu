@@ -314,6 +314,25 @@ static int launch_rolling(FopArgs<R> a, int sign, cudaStream_t st) {
   return nb * NTF;
 }
 
+template <typename R>
+void fop_traces(const Geo& g, int N, const void* Uinv, const void* src, void* trace,
+                cudaStream_t st) {
+  typedef typename CT<R>::T T;
+  FopArgs<R> a = {};
+  a.g = g;
+  a.Uinv = (const T*)Uinv;
+  a.src = (const T*)src;
+  a.trace = (T*)trace;
+  const dim3 nt((g.V + RL_THREADS - 1) / RL_THREADS, NUMLINK + 1);
+  switch (N) {
+    case 2: launch_dep(k_det_traces<2, R, false>, nt, RL_THREADS, st, a); break;
+    case 3: launch_dep(k_det_traces<3, R, false>, nt, RL_THREADS, st, a); break;
+    default: launch_dep(k_det_traces<4, R, false>, nt, RL_THREADS, st, a); break;
+  }
+}
+template void fop_traces<double>(const Geo&, int, const void*, const void*, void*, cudaStream_t);
+template void fop_traces<float>(const Geo&, int, const void*, const void*, void*, cudaStream_t);
+
 // Resident blocks per SM: as many as hold a product's operands, the
 // accumulator and the addresses without spilling (80 / 64 registers for
 // NCOL 2, 128 / 80 for 3, 255 / 128 for 4, FP64 / FP32).  wide: a step fewer,
@@ -425,9 +444,10 @@ int fermion_op_batch(const FopArgs<R>* args, int n, int N, int sign, int chain, 
     FopArgs<R>& a = B.a[i];
     a = args[i];
     if (!a.trace) return -1;
-    if (chain == FOP_FIRST && a.doG) a.trace_out = a.trace + 6 * (size_t)a.g.S;
+    if ((chain == FOP_FIRST || chain == FOP_TRACED) && a.doG)
+      a.trace_out = a.trace + 6 * (size_t)a.g.S;
     if (chain == FOP_SECOND) a.trace += 6 * (size_t)a.g.S;
-    traces = traces || (a.doG && chain != FOP_SECOND);
+    traces = traces || (a.doG && (chain == FOP_ALONE || chain == FOP_FIRST));
     B.start[i] = (int)t;
     t += (a.g.V + RL_THREADS - 1) / RL_THREADS;
   }

@@ -69,6 +69,11 @@ struct MsBlockVecs {
   void* p0_32;
   void* mp32;
   int f32;
+  int N, S;            // NCOL and the site stride
+  // rolling operator with G != 0: U^-1 in the operator's precision and the
+  // trace field the p0 update fills for the next D (else nullptr)
+  const void* Uinv;
+  void* trace;
 };
 
 // fermion_op.cu, fermion_op_rows.cu
@@ -110,7 +115,8 @@ enum { FOP_MAT = 0, FOP_MAT_CM = 1, FOP_ROWS = 2, FOP_COMPACT = 3, FOP_COMPACT_P
 // D and the D^dag that follows it on D's result, with nothing between them on
 // the context: the rolling kernels' D then writes the traces that D^dag reads
 // (the second 6 S complex of the trace field), saving that pre-pass.
-enum { FOP_ALONE = 0, FOP_FIRST = 1, FOP_SECOND = 2 };
+// FOP_TRACED: such a D whose own source's traces are in place already.
+enum { FOP_ALONE = 0, FOP_FIRST = 1, FOP_SECOND = 2, FOP_TRACED = 3 };
 template <typename R>
 int fermion_op(const Geo& g, int N, const void* U, const void* Uinv, const void* pd,
                 const void* src, void* dst, int sign, double G, const void* add, double addc,
@@ -122,6 +128,10 @@ int fermion_op_rows(const FopArgs<R>& a, int N, int sign, cudaStream_t st);
 int fop_partials(const Geo& g);
 template <typename R>
 int fermion_op_rolling(const FopArgs<R>& a, int N, int sign, bool wide, cudaStream_t st);
+// The trace pre-pass of D alone, into the first half of the trace field
+template <typename R>
+void fop_traces(const Geo& g, int N, const void* Uinv, const void* src, void* trace,
+                cudaStream_t st);
 // Its term table on the current device (upload_fop_terms)
 int upload_rolling_terms();
 template <typename R>
@@ -177,7 +187,8 @@ void msb_update_r(MsState* st, const MsBlockVecs& v, long n, double* part, bool 
                   cudaStream_t s);
 void msb_replace(MsState* st, const MsBlockVecs& v, long n, const void* rt, double rsq,
                  cudaStream_t s);
-void msb_update_p0(MsState* st, const MsBlockVecs& v, long n, cudaStream_t s);
+void msb_update_p0(MsState* st, const MsBlockVecs& v, cudaStream_t s);
+int msb_p0_blocks(int S);
 void msb_block(MsState* st, const MsBlockVecs& v, long n, cudaStream_t s);
 void ms_set_stop(MsState* st, double errormin_base, cudaStream_t s);
 
@@ -191,15 +202,17 @@ struct MsLat {
   double* part0;   // operator partials (16 ceil(V / 128) of them)
   int np0;
   double* part1;   // |r|^2 partials, one per block of the residual update
-  int rblk0, rblocks;   // first block and blocks in the residual update's table
-  int vblk0, vblocks;   // and in the other vector kernels' (vec_blocks(n))
+  // first block and blocks in the tables of the residual update
+  // (msbat_rblocks(n)), the p0 update (msb_p0_blocks(S)) and the block pass
+  // (vec_blocks(n))
+  int rblk0, rblocks, qblk0, vblk0;
 };
 int msbat_rblocks(long n);
 // The kernels of the blocked solver for every lattice of a batch at once
-// (L: a device array of nl MsLat; rtot, vtot: table sizes)
+// (L: a device array of nl MsLat; rtot, qtot, vtot: table sizes; N: NCOL)
 void ms_batch_scalars1(const MsLat* L, int nl, cudaStream_t s);
 void ms_batch_update_r(const MsLat* L, int nl, int rtot, cudaStream_t s);
-void ms_batch_update_p0(const MsLat* L, int nl, int vtot, cudaStream_t s);
+void ms_batch_update_p0(const MsLat* L, int nl, int N, int qtot, cudaStream_t s);
 void ms_batch_block(const MsLat* L, int nl, int vtot, cudaStream_t s);
 // out[i] = lattice i's stop flag
 void ms_batch_skips(const MsLat* L, int nl, int* out, cudaStream_t s);

@@ -45,7 +45,9 @@ struct susy_b200_lattice {
   double* meas = nullptr;     // measurement partials
   size_t meas_n = 0;
   int ms_blocked = 1;         // FP64 multi-shift CG: blocked vector update
-  int use_graphs = 1;         // replay the solver's iteration chunks as CUDA graphs
+  int use_graphs = 1;         // susy_b200_use_graphs: 0 = never replay the solver's
+                              // iteration chunks as CUDA graphs
+  int graphs_asked = 0;       // replay them: set by an explicit use_graphs(1)
   int host_solver = 0;        // solver behind susy_b200_congrad_multi
   double mix_switch = 3e-4;   // mixed solver: FP32 operator once |r| < this |src|
   double mix_reliable = 1e-2; // mixed solver: true residual when |r| fell this much
@@ -87,6 +89,9 @@ void refresh_low(susy_b200_lattice* h);
 int dev_fop(susy_b200_lattice* h, const void* src, void* dst, int sign, int prec,
             const void* add, double addc, double* dot, const int* skip,
             int chain = FOP_ALONE);
+// Whether the operator kernel in use reads the trace pre-pass's traces by row
+// (chains D and D^dag); tunes first if need be
+bool fop_uses_traces(susy_b200_lattice* h, int prec);
 int autotune_fop(susy_b200_lattice* h, int prec);
 void* scratch_tf(susy_b200_lattice* h, int which, int prec);
 double* partials(susy_b200_lattice* h, int which);

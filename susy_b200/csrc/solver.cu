@@ -122,7 +122,7 @@ static int ms_run(susy_b200_lattice* h, const void* src, void* const* psim, int 
 // lattices of one NCOL at once.  Every lattice is set up as ms_run_block sets
 // up one solve (its own state, vectors and partials in its handle); then each
 // iteration is five launches for all lattices together: the batched
-// operator D and its trace pre-pass, D^dag with the (fmass^2 + shift_0) p0
+// operator D, D^dag with the (fmass^2 + shift_0) p0
 // epilogue and the <p0, mp> partials, the first recurrences, the residual
 // update with the second recurrences, the p0 update; and every MS_BLK
 // iterations the block pass.  The per-iteration form streamed every live
@@ -136,7 +136,7 @@ static int ms_run_batch(susy_b200_lattice* const* hs, int nl, const void* const*
                         double* size_r, int* iters, cudaStream_t st) {
   std::vector<MsLat> L(nl);
   std::vector<FopArgs<double>> aD(nl), aDd(nl);
-  int vtot = 0, rtot = 0;
+  int vtot = 0, rtot = 0, qtot = 0;
   for (int i = 0; i < nl; i++) {
     susy_b200_lattice* h = hs[i];
     const long n = tf_complex(h);
@@ -159,6 +159,11 @@ static int ms_run_batch(susy_b200_lattice* const* hs, int nl, const void* const*
     v.p0_32 = nullptr;
     v.mp32 = nullptr;
     v.f32 = 0;
+    v.N = h->N;
+    v.S = h->g.S;
+    v.Uinv = h->Uinv;
+    v.trace = h->G > 1e-8 ? h->trace[0] : nullptr;
+    if (v.trace) fop_traces<double>(h->g, h->N, h->Uinv, src[i], v.trace, st);
     // the allocations above zero their fields on h's stream
     if (h->stream != st && cudaStreamSynchronize(h->stream) != cudaSuccess) return SUSY_B200_ECUDA;
     // r(0) = src, p0 = P_j = src, psi_j = 0   (congrad_multi.c:47-57)
@@ -184,9 +189,10 @@ static int ms_run_batch(susy_b200_lattice* const* hs, int nl, const void* const*
     L[i].rblk0 = rtot;
     L[i].rblocks = msbat_rblocks(n);
     rtot += L[i].rblocks;
+    L[i].qblk0 = qtot;
+    qtot += msb_p0_blocks(h->g.S);
     L[i].vblk0 = vtot;
-    L[i].vblocks = vec_blocks(n);
-    vtot += L[i].vblocks;
+    vtot += vec_blocks(n);
   }
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -210,12 +216,12 @@ static int ms_run_batch(susy_b200_lattice* const* hs, int nl, const void* const*
   int launched = 0;
   for (;;) {
     for (int k = 0; k < chunk && !rc; k++) {
-      if (fermion_op_batch<double>(aD.data(), nl, N, 1, FOP_FIRST, sms, st) < 0 ||
+      if (fermion_op_batch<double>(aD.data(), nl, N, 1, FOP_TRACED, sms, st) < 0 ||
           fermion_op_batch<double>(aDd.data(), nl, N, -1, FOP_SECOND, sms, st) < 0)
         rc = SUSY_B200_EINVAL;
       ms_batch_scalars1(dL, nl, st);
       ms_batch_update_r(dL, nl, rtot, st);
-      ms_batch_update_p0(dL, nl, vtot, st);
+      ms_batch_update_p0(dL, nl, N, qtot, st);
       if ((k + 1) % MS_BLK == 0) ms_batch_block(dL, nl, vtot, st);
     }
     launched += chunk;
@@ -366,6 +372,8 @@ static int ms_run_block(susy_b200_lattice* h, const void* src, void* const* psim
   v.p0_32 = nullptr;
   v.mp32 = mp32;
   v.f32 = 0;
+  v.N = h->N;
+  v.S = h->g.S;
   // r(0) = src, p0 = P_j = src, psi_j = 0   (congrad_multi.c:47-57)
   cudaMemcpyAsync(v.ring[0], src, bv, cudaMemcpyDeviceToDevice, s);
   cudaMemcpyAsync(p0, src, bv, cudaMemcpyDeviceToDevice, s);
@@ -385,6 +393,21 @@ static int ms_run_block(susy_b200_lattice* h, const void* src, void* const* psim
   const int chunk = (mixed && h->mix_interval > 0) ? MS_BLK : 2 * MS_BLK;
   double* pd = (double*)(pw + 2);  // pinned: the iterated |r|^2
   bool fp32_op = false;
+  // The p0 update keeps the traces of the operator's input for D; whatever
+  // else writes that field (the start, the switch to FP32, a residual
+  // replacement) calls this after it
+  auto retrace = [&]() {
+    const int prec = fp32_op ? 32 : 64;
+    v.trace = nullptr;
+    if (!(h->G > 1e-8) || !fop_uses_traces(h, prec)) return;
+    v.Uinv = fp32_op ? h->Uinv32 : h->Uinv;
+    v.trace = h->trace[fp32_op ? 1 : 0];
+    if (fp32_op)
+      fop_traces<float>(h->g, h->N, v.Uinv, p0_32, v.trace, s);
+    else
+      fop_traces<double>(h->g, h->N, v.Uinv, p0, v.trace, s);
+  };
+  retrace();
   double bnorm = 0.0, last_true = 0.0, rsqstop = 0.0;
   if (mixed) {
     cudaMemcpyAsync(pd, &h->ms->source_norm, sizeof(double), cudaMemcpyDeviceToHost, s);
@@ -403,15 +426,15 @@ static int ms_run_block(susy_b200_lattice* h, const void* src, void* const* psim
     for (int k = 0; k < chunk; k++) {
       int np_fop;
       if (fp32_op) {
-        dev_fop(h, p0_32, tmp32, 1, 32, nullptr, 0.0, nullptr, skip, FOP_FIRST);
+        dev_fop(h, p0_32, tmp32, 1, 32, nullptr, 0.0, nullptr, skip, FOP_TRACED);
         np_fop = dev_fop(h, tmp32, mp32, -1, 32, p0_32, fm2 + shift[0], part0, skip, FOP_SECOND);
       } else {
-        dev_fop(h, p0, tmp, 1, 64, nullptr, 0.0, nullptr, skip, FOP_FIRST);
+        dev_fop(h, p0, tmp, 1, 64, nullptr, 0.0, nullptr, skip, FOP_TRACED);
         np_fop = dev_fop(h, tmp, mp, -1, 64, p0, fm2 + shift[0], part0, skip, FOP_SECOND);
       }
       ms_scalars1(h->ms, part0, np_fop, s);
       msb_update_r(h->ms, v, n, part1, fp32_op, s);
-      msb_update_p0(h->ms, v, n, s);
+      msb_update_p0(h->ms, v, s);
       if ((k + 1) % MS_BLK == 0) msb_block(h->ms, v, n, s);
     }
   };
@@ -440,16 +463,23 @@ static int ms_run_block(susy_b200_lattice* h, const void* src, void* const* psim
       // update
       v.p0_32 = p0_32;
     }
+    retrace();
     return true;
   };
   // fp32_below = 1: the FP32 operator from the first iteration
   if (mixed && h->mix_switch >= 1.0 && !to_fp32(0)) return set_err(h, SUSY_B200_ENOMEM);
-  // A chunk's ~100 launches are captured once per operator precision into a
-  // CUDA graph and replayed: every argument of them is fixed for the solve
-  // (the convergence test and the freezing of shifts read device state).
+  // A caller that asked for graphs gets a chunk's ~80 launches captured once
+  // per operator precision and replayed: every argument of them is fixed for
+  // the solve (the convergence test and the freezing of shifts read device
+  // state).  Otherwise they are launched: programmatic dependent launches are
+  // issued faster than they run, and capturing and instantiating cost each
+  // solve 0.2 to 0.4 ms (4^4 U(2) solve 2.92 ms with graphs, 2.71 without;
+  // 4^4 trajectory 44.8 and 42.6, with two pseudofermions 58.8 and 52.0; 24
+  // lattices' trajectories on 24 threads 503 and 451 ms).
+  const bool replay = h->use_graphs && h->graphs_asked;
   ChunkGraph graphs[2];
   for (;;) {
-    if (h->use_graphs) {
+    if (replay && h->use_graphs) {
       ChunkGraph& cg = graphs[fp32_op ? 1 : 0];
       if (!cg.ready) cg.capture(h, fp32_op ? 32 : 64, issue_chunk);
       if (cg.ready)
@@ -492,6 +522,7 @@ static int ms_run_block(susy_b200_lattice* h, const void* src, void* const* psim
         if (trace) fprintf(stderr, "susy_b200 cg: reliable update at %d: true rsq %.6e\n", it, rt);
         if (!(rt == rt)) return set_err(h, SUSY_B200_ENAN);
         msb_replace(h->ms, v, n, rt64, rt, s);
+        retrace();
         last_true = rt;
         last_rel = it;
         replacements++;
