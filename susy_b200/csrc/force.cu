@@ -26,7 +26,7 @@ struct FfArgs {
   const double2 *Uinv, *pd;
   const double2 *sol, *psol;  // psol = D sol (not yet scaled by amp)
   double2* force;             // accumulates amp * f_U^dag
-  const double2* tr;          // traces of k_ff_traces, [12][S]
+  const double2* tr;          // traces of sol and psol, [12][S] (k_ff_traces)
   const int* nbrtab;          // the operator's neighbour index table
   double amp, G;
   int doG;
@@ -106,16 +106,19 @@ int upload_force_terms() {
 
 // Every trace detF needs, once per site instead of once per link that reads
 // it (up to 20 of two matrices each per link and source before):
-//   tr[e] = Tr U_e^-1 psi_e, tr[5 + e] = Tr U_e^-1 psi'_e^dag,
-//   tr[10] = Tr eta, tr[11] = conj Tr eta'
-// (psi, eta of sol, primed of psol).  One thread per site and e = blockIdx.y;
-// e = 5 the two of the site component.
+//   tr[e] = Tr U_e^-1 psi_e, tr[5] = Tr eta,
+//   tr[6 + e] = Tr U_e^-1 psi'_e^dag, tr[11] = conj Tr eta'
+// (psi, eta of sol, primed of psol).  The rolling operator kernels leave
+// exactly these in their trace field when they form psol = D sol; this
+// pre-pass (19 us a pole at 12^3x24 U(3)) serves the other kernels.  One thread
+// per site and e = blockIdx.y; e = 5 the two of the site component.
 template <int N>
 __global__ void __launch_bounds__(FT) k_ff_traces(FfArgs a, double2* tr) {
+  wait_prior();
   const int s = blockIdx.x * FT + threadIdx.x, e = blockIdx.y, S = a.g.S;
   if (s >= a.g.V) return;
   if (e == NUMLINK) {
-    stc<double>(tr + (size_t)10 * S + s, ldtr<N, double, false>(a.sol, 0, s, S));
+    stc<double>(tr + (size_t)5 * S + s, ldtr<N, double, false>(a.sol, 0, s, S));
     stc<double>(tr + (size_t)11 * S + s, ldtr<N, double, true>(a.psol, 0, s, S));
     return;
   }
@@ -132,7 +135,7 @@ __global__ void __launch_bounds__(FT) k_ff_traces(FfArgs a, double2* tr) {
       t1 = t1 + u * conj(ldc<double>(pp + (size_t)(i * N + k) * S));
     }
   stc<double>(tr + (size_t)e * S + s, t0);
-  stc<double>(tr + (size_t)(5 + e) * S + s, t1);
+  stc<double>(tr + (size_t)(6 + e) * S + s, t1);
 }
 
 // One direction b's share of detF (update_h.c:477-651), for both of its
@@ -160,9 +163,9 @@ SUSY_D void ff_det(const FfArgs& a, const Site& c, int M, int b, Cx<double>& u, 
 #pragma unroll
   for (int q = 0; q < 2; q++) {
     const double localG = (q == 0 ? -0.5 : 0.5) * a.G;
-    const double2* te = a.tr + (size_t)(q == 0 ? 11 : 10) * S;
-    const double2* TM = a.tr + (size_t)(5 * q + M) * S;
-    const double2* Tb = a.tr + (size_t)(5 * q + b) * S;
+    const double2* te = a.tr + (size_t)(q == 0 ? 11 : 5) * S;
+    const double2* TM = a.tr + (size_t)(6 * q + M) * S;
+    const double2* Tb = a.tr + (size_t)(6 * q + b) * S;
     const Cx<double> te0 = ldc<double>(te + s), te_mb = ldc<double>(te + mb);
     const Cx<double> TM0 = ldc<double>(TM + s);
     const Cx<double> DbM = te0 * bM, DMb = te0 * Mb;
@@ -210,6 +213,7 @@ template <int N>
 __global__ void __launch_bounds__(FT, ff_blocks<N>()) k_fermion_force(FfArgs a) {
   __shared__ double2 sacc[3][N * N][32];
   __shared__ double2 sdet[4][3][32];
+  wait_prior();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int M = blockIdx.x % NUMLINK;
   const int s = (blockIdx.x / NUMLINK) * 32 + lane;
@@ -516,15 +520,15 @@ int force_blocks(const Geo& g) { return nbk(g.V, FT) * NUMLINK; }
 int site_blocks(const Geo& g) { return nbk(g.V, FT); }
 
 template <int N>
-static void launch_fermion_force(const FfArgs& a, double2* tr, cudaStream_t st) {
-  if (a.doG)
-    count_launch(), k_ff_traces<N><<<dim3(nbk(a.g.V, FT), NUMLINK + 1), FT, 0, st>>>(a, tr);
-  count_launch(), k_fermion_force<N><<<nbk(a.g.V, 32) * NUMLINK, FT, 0, st>>>(a);
+static void launch_fermion_force(const FfArgs& a, double2* tr, bool traced, cudaStream_t st) {
+  if (a.doG && !traced)
+    launch_dep(k_ff_traces<N>, dim3(nbk(a.g.V, FT), NUMLINK + 1), FT, st, a, tr);
+  launch_dep(k_fermion_force<N>, nbk(a.g.V, 32) * NUMLINK, FT, st, a);
 }
 
 void fermion_force_pole(const Geo& g, int N, const void* Uinv, const void* pd,
                         const void* sol, const void* psol, void* force, void* tr,
-                        const int* nbrtab, double amp, double G, cudaStream_t st) {
+                        bool traced, const int* nbrtab, double amp, double G, cudaStream_t st) {
   FfArgs a;
   a.g = g;
   a.Uinv = (const double2*)Uinv;
@@ -538,9 +542,9 @@ void fermion_force_pole(const Geo& g, int N, const void* Uinv, const void* pd,
   a.G = G;
   a.doG = G > 1e-8;
   switch (N) {
-    case 2: launch_fermion_force<2>(a, (double2*)tr, st); break;
-    case 3: launch_fermion_force<3>(a, (double2*)tr, st); break;
-    case 4: launch_fermion_force<4>(a, (double2*)tr, st); break;
+    case 2: launch_fermion_force<2>(a, (double2*)tr, traced, st); break;
+    case 3: launch_fermion_force<3>(a, (double2*)tr, traced, st); break;
+    case 4: launch_fermion_force<4>(a, (double2*)tr, traced, st); break;
   }
 }
 

@@ -131,13 +131,15 @@ int dev_fermion_force(susy_b200_lattice* h, double eps, void* const* sol, int no
                       const double* amp4, double* norm) {
   void* psol = scratch_tf(h, 2, 64);
   double* part = big_partials(h);
-  if (!h->ftrace) h->ftrace = dalloc(h, 12L * h->g.S * sizeof(double2));
-  if (!psol || !part || !h->ftrace) return SUSY_B200_ENOMEM;
+  const bool traced = fop_uses_traces(h, 64);
+  if (!traced && !h->ftrace) h->ftrace = dalloc(h, 12L * h->g.S * sizeof(double2));
+  void* tr = traced ? h->trace[0] : h->ftrace;
+  if (!psol || !part || !tr) return SUSY_B200_ENOMEM;
   cudaMemsetAsync(h->force, 0, field_bytes(h, 5, 64), h->stream);
   for (int n = 0; n < norder; n++) {
-    dev_fop(h, sol[n], psol, 1, 64, nullptr, 0.0, nullptr, nullptr);
-    fermion_force_pole(h->g, h->N, h->Uinv, h->pd, sol[n], psol, h->force, h->ftrace, h->nbrtab,
-                       amp4[n], h->G, h->stream);
+    dev_fop(h, sol[n], psol, 1, 64, nullptr, 0.0, nullptr, nullptr, FOP_FIRST);
+    fermion_force_pole(h->g, h->N, h->Uinv, h->pd, sol[n], psol, h->force, tr, traced,
+                       h->nbrtab, amp4[n], h->G, h->stream);
   }
   const int nb = mom_sub(mat5(h), h->force, h->mom, eps, part, h->stream);
   if (!ck(h, cudaGetLastError())) return SUSY_B200_ECUDA;

@@ -225,10 +225,11 @@ int force_blocks(const Geo& g);
 int site_blocks(const Geo& g);
 // The fermion force's term table on the current device (upload_fop_terms)
 int upload_force_terms();
-// force += amp f_U^dag of one pole; tr: 12 S complex of scratch
+// force += amp f_U^dag of one pole; tr: 12 S complex, the operator's trace
+// field with the traces of sol and psol in it (traced) or scratch
 void fermion_force_pole(const Geo& g, int N, const void* Uinv, const void* pd,
                         const void* sol, const void* psol, void* force, void* tr,
-                        const int* nbrtab, double amp, double G, cudaStream_t st);
+                        bool traced, const int* nbrtab, double amp, double G, cudaStream_t st);
 int mom_sub(long n, const void* force, void* mom, double eps, double* part, cudaStream_t st);
 void axpy_field(long n, double s, const void* x, void* y, cudaStream_t st);
 int gauge_force(const Geo& g, int N, const void* U, const void* Uinv, const void* pd,
