@@ -365,8 +365,8 @@ void susy_b200_destroy(susy_b200_lattice* h) {
   }
   for (int i = 0; i < SUSY_NPART; i++)
     if (h->part[i]) cudaFree(h->part[i]);
-  for (std::vector<void*>* v : {&h->extra, &h->sols, &h->pvec64, &h->pvec32, &h->ring, &h->vec32, &h->gsrc,
-                                &h->gr_psim, &h->traj_psim, &h->extra5, &h->refine})
+  for (std::vector<void*>* v : {&h->extra, &h->sols, &h->gsrc, &h->gr_psim,
+                                &h->traj_psim, &h->extra5, &h->refine})
     for (void* p : *v)
       if (p) cudaFree(p);
   if (h->poll) cudaFreeHost(h->poll);

@@ -565,9 +565,8 @@ SUSY_D void update_r_block(MsState* st, const MsBlockVecs& v, long n, double* pa
 }
 
 template <typename MT, typename RT>
-// six blocks per SM: the coefficient step of the last block must not cost the
-// streaming loop its occupancy (58 us a launch at 12^3x24 U(3) with four, 51
-// with six)
+// six blocks per SM: the coefficient step of the last block must not take the
+// streaming loop's registers (40 instead of 58; the step itself spills)
 __global__ void __launch_bounds__(UT, 6) k_msb_update_r(MsState* st, MsBlockVecs v, long n,
                                                         double* part) {
   wait_prior();

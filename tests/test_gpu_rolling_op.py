@@ -37,3 +37,38 @@ def test_rolling_operator(dims, N, pbc, G, fmass):
             lat.dev_DSq(a, b)
             got = synth.from_ref(dims, b.download(), 16, N)
             assert np.abs(got - want).max() <= tol * np.abs(want).max()
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("maxcg,zero", [(3, False), (8, False), (5000, False), (5000, True)])
+def test_solver_chained_through_the_rolling_operator(maxcg, zero, mixed):
+    """The solver's p0 update leaves D's traces and D those of D^dag: the same
+    iterations and solutions as with an operator kernel that reads none
+    (FOP_SITE_MAJOR_FRONT), when the solve stops inside a block of 8, at its
+    end, by convergence, and at once (zero source)."""
+    dims, N = (4, 4, 2, 10), 3
+    lat = Lattice(dims, N, pbc=-1, lam=1.0, bmass=0.2, G=0.05)
+    lat.set_links(synth.to_ref(dims, synth.links(dims, N, 0.2, 7)))
+    src = lat.tf(64)
+    host = synth.to_ref(dims, synth.tf_source(dims, N, seed=21))
+    src.upload(np.zeros_like(host) if zero else host)
+    shifts = synth.geometric_shifts(5, 1e-3, 1e2)
+    out = {}
+    for v in (12,) + ROLLING:
+        lat.fop_variant(64, v)
+        lat.fop_variant(32, v)
+        psim = [lat.tf(64) for _ in shifts]
+        # the truncated solves compare plain FP64 iterations
+        it, _ = lat.dev_congrad_multi(src, psim, shifts, maxcg, 1e-20, mixed=mixed and maxcg > 8)
+        out[v] = (it, [p.download() for p in psim])
+    # a converged solution is fixed to residual / smallest eigenvalue of the
+    # shifted operator, 1e-10 |src| / 1e-3; a truncated one to the rounding of
+    # its few iterations
+    tol = 1e-7 * np.linalg.norm(host) if maxcg > 8 else 1e-11 * np.linalg.norm(host)
+    for v in ROLLING:
+        if not mixed:
+            assert abs(out[v][0] - out[12][0]) <= 1
+        if zero:
+            assert out[v][0] == 0
+        for a, b in zip(out[v][1], out[12][1]):
+            assert np.isfinite(a).all() and np.linalg.norm(a - b) <= tol
