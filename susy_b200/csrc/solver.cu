@@ -177,9 +177,11 @@ static int ms_run_batch(susy_b200_lattice* const* hs, int nl, const void* const*
     v.S = h->g.S;
     v.Uinv = h->Uinv;
     v.trace = h->G > 1e-8 ? h->trace[0] : nullptr;
-    if (v.trace) fop_traces<double>(h->g, h->N, h->Uinv, src[i], v.trace, st);
-    // the allocations above zero their fields on h's stream
+    // Work still queued on h's stream may be writing src[i] or the links'
+    // inverses, or reading the trace field, and the allocations above zero
+    // their fields there: nothing of this lattice goes to st before it is done
     if (h->stream != st && cudaStreamSynchronize(h->stream) != cudaSuccess) return SUSY_B200_ECUDA;
+    if (v.trace) fop_traces<double>(h->g, h->N, h->Uinv, src[i], v.trace, st);
     // r(0) = src, p0 = P_j = src, psi_j = 0   (congrad_multi.c:47-57)
     cudaMemcpyAsync(v.ring[0], src[i], bv, cudaMemcpyDeviceToDevice, st);
     cudaMemcpyAsync(p0, src[i], bv, cudaMemcpyDeviceToDevice, st);

@@ -73,3 +73,54 @@ def test_batch_solve_refuses_a_handle_twice_and_bad_counts():
     with pytest.raises(SusyError):
         congrad_multi_batch([src], [[lat.tf(64) for _ in range(33)]],
                             [synth.geometric_shifts(33, 1e-3, 1.0)], 100, 1e-16)
+
+
+def true_residuals(lat, b, psim, shifts, fm):
+    """|b - (D^dag D + fm^2 + sigma_j) psi_j|^2 / |b|^2 of every shift, with an
+    operator kernel that reads no traces"""
+    lat.fop_variant(64, FRONT)
+    ap, nb = lat.tf(64), np.linalg.norm(b) ** 2
+    out = []
+    for p, s in zip(psim, shifts):
+        lat.dev_DSq(p, ap)          # fmass^2 included
+        x, ax = p.download(), ap.download()
+        out.append(np.linalg.norm(b - ax - s * x) ** 2 / nb)
+    return out
+
+
+@pytest.mark.parametrize("cuda_stream", ["first handle's", "the caller's"])
+def test_batch_solve_waits_for_each_handles_own_stream(cuda_stream):
+    """New links and a new source set on handles with streams of their own,
+    the source behind a queue of operator applications, and the batched solve
+    called at once: it must solve with the new ones.  The trace field D reads
+    first is filled from both, so traces of the old ones leave the iterated
+    residual converged and the true one not.  Bound on the true residual: the
+    drift of the iterated one is eps |A| |x| an iteration, with |A| <= 50 and
+    |x| <= |b| / 1e-2 at most 1e-12 |b|; 1000 iterations of it all in one
+    direction stay below 1e-9 |b|, 1e-18 squared."""
+    import torch
+    dims, shifts, fm = (8, 8, 8, 8), synth.geometric_shifts(4, 1e-2, 1e2), 0.0
+    lats, srcs, psims, tmp, firsts = [], [], [], [], []
+    st = torch.cuda.Stream()
+    for k in range(3):
+        lat = Lattice(dims, 2, pbc=-1, lam=1.0, bmass=0.2, G=0.1, fmass=fm)
+        lat.fop_variant(64, 10)
+        src, first = lat.tf(64), lat.tf(64)
+        first.upload(synth.to_ref(dims, synth.tf_source(dims, 2, 90 + k)))
+        lats.append(lat)
+        srcs.append(src)
+        firsts.append(first)
+        tmp.append(lat.tf(64))
+        psims.append([lat.tf(64) for _ in shifts])
+    args = (5000, 1e-20) + ((st.cuda_stream,) if cuda_stream == "the caller's" else ())
+    for rnd in range(2):                # the second finds every field allocated
+        for k, lat in enumerate(lats):
+            lat.set_links(synth.to_ref(dims, synth.links(dims, 2, 0.2, 40 + 10 * rnd + k)))
+            for _ in range(100 * 3 ** k):
+                lat.dev_DSq(firsts[k], tmp[k])
+            lat.dev_convert(tmp[k], srcs[k])
+        congrad_multi_batch(srcs, psims, [shifts] * 3, *args)
+        for k, lat in enumerate(lats):
+            res = true_residuals(lat, srcs[k].download(), psims[k], shifts, fm)
+            assert max(res) <= 1e-18, (rnd, k, res)
+            lat.fop_variant(64, 10)
