@@ -611,7 +611,7 @@ SUSY_D void msb_p0_block(const MsState* st, const MsBlockVecs& v, int blk) {
 #pragma unroll
     for (int i = 0; i < N; i++)
 #pragma unroll
-      for (int j = 0; j < N; j++) t = t + ldc<OR>(pu + (long)(i * N + j) * v.S) * m.e[j][i];
+      for (int j = 0; j < N; j++) t = t + ldv<OR>(pu + (long)(i * N + j) * v.S) * m.e[j][i];
   }
   stc<OR>((T*)v.trace + (long)(k == 0 ? NUMLINK : k - 1) * v.S + s, t);
 }

@@ -82,11 +82,11 @@ struct LinkPtr {
 // left to the use: a sign here would wait for the load)
 template <int N, typename R, bool ADJF>
 SUSY_D Cx<R> ld_src(const typename CT<R>::T* p, int i, int j, int S) {
-  return ldc<R>(p + (size_t)((ADJF ? j * N + i : i * N + j) * S));
+  return ldv<R>(p + (size_t)((ADJF ? j * N + i : i * N + j) * S));
 }
 template <typename R>
 SUSY_D Cx<R> ld_link(const LinkPtr<R>& u, int i, int j) {
-  return ldc<R>(u.p + i * u.si + j * u.sj);
+  return ldv<R>(u.p + i * u.si + j * u.sj);
 }
 
 // acc += op(U) F (UF) or F op(U), op(U)'s elements times (c, ci) as they are
@@ -146,12 +146,12 @@ SUSY_D void rl_det_site(Mat<N, R>& acc, const FopArgs<R>& a, const Site& c) {
   for (int b = 0; b < NUMLINK; b++) {
     const int pb = nbr(a.g, c, ex(b), ey(b), ez(b), et(b));
     const R bcb = bcf<R>(a.g, c, et(b));
-    const Cx<R> Tb = ldc<R>(a.trace + (size_t)b * S + s);
+    const Cx<R> Tb = ldv<R>(a.trace + (size_t)b * S + s);
 #pragma unroll
     for (int k = 1; k < NUMLINK; k++) {
       const int e = b + k < NUMLINK ? b + k : b + k - NUMLINK;
-      const Cx<R> Te = ldc<R>(a.trace + (size_t)e * S + pb);
-      sum = sum + ldc<R>(a.pd + (size_t)(e * 5 + b) * S + s) * (Tb + bcb * Te);
+      const Cx<R> Te = ldv<R>(a.trace + (size_t)e * S + pb);
+      sum = sum + ldv<R>(a.pd + (size_t)(e * 5 + b) * S + s) * (Tb + bcb * Te);
     }
   }
   const Cx<R> d = ((R)0.5 * a.G) * sum;
@@ -162,21 +162,21 @@ template <int N, typename R>
 SUSY_D void rl_det_link(Mat<N, R>& acc, const FopArgs<R>& a, const Site& c, int B) {
   const int S = a.g.S, s = c.s;
   const typename CT<R>::T* te = a.trace + (size_t)5 * S;
-  const Cx<R> te0 = ldc<R>(te + s);
+  const Cx<R> te0 = ldv<R>(te + s);
   Cx<R> sum(0, 0);
 #pragma unroll
   for (int k = 1; k < NUMLINK; k++) {
     const int e = B + k < NUMLINK ? B + k : B + k - NUMLINK;
     const int me = nbr(a.g, c, -ex(e), -ey(e), -ez(e), -et(e));
-    sum = sum + te0 * ldc<R>(a.pd + (size_t)(e * 5 + B) * S + s);
-    sum = sum + bcf<R>(a.g, c, -et(e)) * (ldc<R>(te + me) * ldc<R>(a.pd + (size_t)(B * 5 + e) * S + me));
+    sum = sum + te0 * ldv<R>(a.pd + (size_t)(e * 5 + B) * S + s);
+    sum = sum + bcf<R>(a.g, c, -et(e)) * (ldv<R>(te + me) * ldv<R>(a.pd + (size_t)(B * 5 + e) * S + me));
   }
   const Cx<R> d = ((R)(-0.5) * a.G * a.eta_scale) * sum;
   const typename CT<R>::T* pu = a.Uinv + (size_t)(B * N * N) * S + s;
 #pragma unroll
   for (int i = 0; i < N; i++)
 #pragma unroll
-    for (int j = 0; j < N; j++) cfma(acc.e[i][j], d, ldc<R>(pu + (size_t)(i * N + j) * S));
+    for (int j = 0; j < N; j++) cfma(acc.e[i][j], d, ldv<R>(pu + (size_t)(i * N + j) * S));
 }
 
 // Output component comp at site s0 (lanes past the volume compute and drop its
@@ -263,7 +263,7 @@ SUSY_D double rl_site(const FopArgs<R>& a, int comp, int s0) {
         for (int j = 0; j < N; j++) acc.e[i][j] = Cx<R>(-m.e[j][i].re, m.e[j][i].im);
     }
     if (a.add) {
-      const Mat<N, R> x = ldm<N, R>(a.add, comp, s, S);
+      const Mat<N, R> x = ldm<N, R, false, true>(a.add, comp, s, S);
       axpy(acc, Cx<R>(a.addc, 0), x);
       if (a.dot) part = rdot(x, acc);
     }
@@ -280,7 +280,7 @@ SUSY_D double rl_site(const FopArgs<R>& a, int comp, int s0) {
         for (int i = 0; i < N; i++)
 #pragma unroll
           for (int j = 0; j < N; j++)
-            t = t + ldc<R>(pu + (size_t)(i * N + j) * S) * conj(acc.e[i][j]);
+            t = t + ldv<R>(pu + (size_t)(i * N + j) * S) * conj(acc.e[i][j]);
       }
       stc<R>(a.trace_out + (size_t)(comp == 0 ? NUMLINK : comp - 1) * S + s, t);
     }

@@ -152,7 +152,7 @@ SUSY_D R bc_of(unsigned mask, int dt, R pbc) {
 // fb at site sb (op(B) = B^dag when ADJB), one element pair at a time: the
 // determinant terms run while the accumulator is live, and holding whole
 // matrices here made the register-capped kernels spill
-template <int N, typename R, bool ADJB>
+template <int N, typename R, bool ADJB, bool DEP = false>
 SUSY_D Cx<R> trace_ld(const typename CT<R>::T* fa, int ka, int sa, const typename CT<R>::T* fb,
                       int kb, int sb, int S) {
   const typename CT<R>::T* pa = fa + (size_t)(ka * N * N) * S + sa;
@@ -162,9 +162,9 @@ SUSY_D Cx<R> trace_ld(const typename CT<R>::T* fa, int ka, int sa, const typenam
   for (int i = 0; i < N; i++)
 #pragma unroll
     for (int k = 0; k < N; k++) {
-      const Cx<R> x = ldc<R>(pa + (size_t)(i * N + k) * S);
-      const Cx<R> y = ADJB ? conj(ldc<R>(pb + (size_t)(i * N + k) * S))
-                           : ldc<R>(pb + (size_t)(k * N + i) * S);
+      const Cx<R> x = ldv<R, DEP>(pa + (size_t)(i * N + k) * S);
+      const Cx<R> y = ADJB ? conj(ldv<R, DEP>(pb + (size_t)(i * N + k) * S))
+                           : ldv<R, DEP>(pb + (size_t)(k * N + i) * S);
       t = t + x * y;
     }
   return t;
@@ -242,8 +242,8 @@ template <int N, typename R, bool ADJ>
 SUSY_D void det_traces_site(const FopArgs<R>& a, int s, int e) {
   if (s >= a.g.V) return;
   const int S = a.g.S;
-  const Cx<R> t = e == NUMLINK ? ldtr<N, R, ADJ>(a.src, 0, s, S)
-                               : trace_ld<N, R, ADJ>(a.Uinv, e, s, a.src, 1 + e, s, S);
+  const Cx<R> t = e == NUMLINK ? ldtr<N, R, ADJ, true>(a.src, 0, s, S)
+                               : trace_ld<N, R, ADJ, true>(a.Uinv, e, s, a.src, 1 + e, s, S);
   stc<R>(a.trace + (size_t)e * S + s, t);
 }
 template <int N, typename R, bool ADJ>

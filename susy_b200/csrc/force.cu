@@ -118,8 +118,8 @@ __global__ void __launch_bounds__(FT) k_ff_traces(FfArgs a, double2* tr) {
   const int s = blockIdx.x * FT + threadIdx.x, e = blockIdx.y, S = a.g.S;
   if (s >= a.g.V) return;
   if (e == NUMLINK) {
-    stc<double>(tr + (size_t)5 * S + s, ldtr<N, double, false>(a.sol, 0, s, S));
-    stc<double>(tr + (size_t)11 * S + s, ldtr<N, double, true>(a.psol, 0, s, S));
+    stc<double>(tr + (size_t)5 * S + s, ldtr<N, double, false, true>(a.sol, 0, s, S));
+    stc<double>(tr + (size_t)11 * S + s, ldtr<N, double, true, true>(a.psol, 0, s, S));
     return;
   }
   const double2* pu = a.Uinv + (size_t)(e * N * N) * S + s;
@@ -130,9 +130,9 @@ __global__ void __launch_bounds__(FT) k_ff_traces(FfArgs a, double2* tr) {
   for (int i = 0; i < N; i++)
 #pragma unroll
     for (int k = 0; k < N; k++) {
-      const Cx<double> u = ldc<double>(pu + (size_t)(i * N + k) * S);
-      t0 = t0 + u * ldc<double>(ps + (size_t)(k * N + i) * S);
-      t1 = t1 + u * conj(ldc<double>(pp + (size_t)(i * N + k) * S));
+      const Cx<double> u = ldv<double>(pu + (size_t)(i * N + k) * S);
+      t0 = t0 + u * ldv<double>(ps + (size_t)(k * N + i) * S);
+      t1 = t1 + u * conj(ldv<double>(pp + (size_t)(i * N + k) * S));
     }
   stc<double>(tr + (size_t)e * S + s, t0);
   stc<double>(tr + (size_t)(6 + e) * S + s, t1);
@@ -157,8 +157,8 @@ SUSY_D void ff_det(const FfArgs& a, const Site& c, int M, int b, Cx<double>& u, 
   const double bcM_mb = bcf<double>(g, cm, et(M));
   const double2* pbM = a.pd + (size_t)(b * 5 + M) * S;
   const double2* pMb = a.pd + (size_t)(M * 5 + b) * S;
-  const Cx<double> bM = ldc<double>(pbM + s), Mb = ldc<double>(pMb + s);
-  const Cx<double> Mb_m = ldc<double>(pMb + mb), bM_m = ldc<double>(pbM + mb);
+  const Cx<double> bM = ldv<double>(pbM + s), Mb = ldv<double>(pMb + s);
+  const Cx<double> Mb_m = ldv<double>(pMb + mb), bM_m = ldv<double>(pbM + mb);
   u = Cx<double>(0, 0);
 #pragma unroll
   for (int q = 0; q < 2; q++) {
@@ -166,14 +166,14 @@ SUSY_D void ff_det(const FfArgs& a, const Site& c, int M, int b, Cx<double>& u, 
     const double2* te = a.tr + (size_t)(q == 0 ? 11 : 5) * S;
     const double2* TM = a.tr + (size_t)(6 * q + M) * S;
     const double2* Tb = a.tr + (size_t)(6 * q + b) * S;
-    const Cx<double> te0 = ldc<double>(te + s), te_mb = ldc<double>(te + mb);
-    const Cx<double> TM0 = ldc<double>(TM + s);
+    const Cx<double> te0 = ldv<double>(te + s), te_mb = ldv<double>(te + mb);
+    const Cx<double> TM0 = ldv<double>(TM + s);
     const Cx<double> DbM = te0 * bM, DMb = te0 * Mb;
     const Cx<double> DMb_mb = te_mb * Mb_m, DbM_mb = te_mb * bM_m;
-    Cx<double> plaq = DbM * (TM0 + bcM * ldc<double>(Tb + pM));
-    plaq = plaq + DMb_mb * (ldc<double>(Tb + mb) + bcmb * TM0);
-    Cx<double> adjt = DMb * (ldc<double>(Tb + s) + bcb * ldc<double>(TM + pb));
-    adjt = adjt + DbM_mb * (ldc<double>(TM + mb) + bcM_mb * ldc<double>(Tb + mbpM));
+    Cx<double> plaq = DbM * (TM0 + bcM * ldv<double>(Tb + pM));
+    plaq = plaq + DMb_mb * (ldv<double>(Tb + mb) + bcmb * TM0);
+    Cx<double> adjt = DMb * (ldv<double>(Tb + s) + bcb * ldv<double>(TM + pb));
+    adjt = adjt + DbM_mb * (ldv<double>(TM + mb) + bcM_mb * ldv<double>(Tb + mbpM));
     u = u + localG * plaq + conj(localG * adjt);
     inv[q] = (-localG) * (DbM + bcmb * DMb_mb);
   }
@@ -189,8 +189,8 @@ SUSY_D void ff_pattern(Mat<N, double>& acc, const FfArgs& a, int s, unsigned bcm
   for (int t = 0; t < FF_ROWS; t++) {
     const FfTerm T = c_ff[M][PAT][t];
     const int il = a.nbrtab[(size_t)T.dl * S + s], ir = a.nbrtab[(size_t)T.dr * S + s];
-    const Mat<N, double> L = ldm<N, double, AL>(SL ? a.sol : a.psol, T.kl, il, S);
-    const Mat<N, double> R = ldm<N, double, !AL>(SL ? a.psol : a.sol, T.kr, ir, S);
+    const Mat<N, double> L = ldm<N, double, AL, true>(SL ? a.sol : a.psol, T.kl, il, S);
+    const Mat<N, double> R = ldm<N, double, !AL, true>(SL ? a.psol : a.sol, T.kr, ir, S);
     mac<0>(acc, T.coef * bc_of<double>(bcm, T.b1, pbc) * bc_of<double>(bcm, T.b2, pbc), L, R);
   }
 }
@@ -267,14 +267,14 @@ __global__ void __launch_bounds__(FT, ff_blocks<N>()) k_fermion_force(FfArgs a) 
     // of the first product at a time; acc holds f^dag
     const double2* ps = a.sol + (size_t)((1 + M) * N * N) * S + s;
     const double2* pp = a.psol + (size_t)((1 + M) * N * N) * S + s;
-    Mat<N, double> ui = ldm<N, double>(a.Uinv, M, s, S);
+    Mat<N, double> ui = ldm<N, double, false, true>(a.Uinv, M, s, S);
     Mat<N, double> w;
 #pragma unroll
     for (int i = 0; i < N; i++)
 #pragma unroll
       for (int j = 0; j < N; j++)
-        w.e[i][j] = d[1] * ldc<double>(ps + (size_t)(i * N + j) * S) +
-                    d[2] * conj(ldc<double>(pp + (size_t)(j * N + i) * S));
+        w.e[i][j] = d[1] * ldv<double>(ps + (size_t)(i * N + j) * S) +
+                    d[2] * conj(ldv<double>(pp + (size_t)(j * N + i) * S));
 #pragma unroll
     for (int i = 0; i < N; i++) {
       Cx<double> row[N];

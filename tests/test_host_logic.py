@@ -118,3 +118,53 @@ def test_bench_quotes_ncu_traffic_only_for_captured_variants():
     # DRAM traffic of a real capture: near the algorithmic bytes, not far below
     assert 0.9 * alg64 < t64 < 2.0 * alg64 and 0.9 * alg32 < t32 < 2.0 * alg32
     assert bench.committed_traffic(0, 1) == (None, None)
+
+
+def _dependent_code():
+    """{name: source} of the device code that launch_dep's kernels run, found
+    from the kernels that call wait_prior() and the functions they call."""
+    import re
+    csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
+                        "susy_b200", "csrc")
+    funcs, launched = {}, set()
+    for f in sorted(os.listdir(csrc)):
+        if not f.endswith((".cu", ".cuh")):
+            continue
+        src = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, f)).read())
+        src = re.sub(r"__launch_bounds__\((?:[^()]|\(\))*\)", "", src)
+        launched |= set(re.findall(r"launch_dep\(\s*(\w+)", src)) - {"void"}
+        for m in re.finditer(r"(?:SUSY_D|__global__)[^;{}=]*?(\w+)\s*\([^;{}]*\)\s*\{", src):
+            depth, i = 1, m.end()
+            while depth:
+                depth += {"{": 1, "}": -1}.get(src[i], 0)
+                i += 1
+            funcs.setdefault(m.group(1), "")
+            funcs[m.group(1)] += src[m.end():i]
+    waiting = {k for k, v in funcs.items() if "wait_prior()" in v}
+    assert launched <= waiting
+    todo, seen = list(waiting), set()
+    while todo:
+        k = todo.pop()
+        if k in seen:
+            continue
+        seen.add(k)
+        todo += [c for c in set(re.findall(r"\b(\w+)\s*(?:<[^;(){}]*>)?\(", funcs[k]))
+                 if c in funcs]
+    return {k: funcs[k] for k in seen}
+
+
+def test_dependent_kernels_read_fields_with_ordinary_loads():
+    """A kernel that may start before the one before it has finished writing
+    must not read through the read-only path (ldc, __ldg): such a load is not
+    held behind the wait.  ldm, ldtr and trace_ld take the load's kind."""
+    import re
+    code = _dependent_code()
+    assert {"fermion_op_rolling_kernel", "rl_site", "det_traces_site", "msb_p0_block",
+            "ff_pattern", "ff_det", "k_fermion_force"} <= set(code)
+    generic = {"ldv", "ldc", "ldm", "ldtr", "trace_ld"}
+    for name, src in code.items():
+        if name in generic:
+            continue
+        assert "__ldg" not in src and not re.search(r"\bldc\s*<", src), name
+        for call in re.findall(r"\b(?:ldm|ldtr|trace_ld)\s*<([^>]*)>", src):
+            assert call.replace(" ", "").endswith(",true") and call.count(",") == 3, (name, call)
