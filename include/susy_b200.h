@@ -173,12 +173,11 @@ int susy_b200_cg_blocked(susy_b200_lattice *h, int on);
  * iteration at which shift j froze, the solve's iteration count for the
  * base shift and for shifts that never froze.  1 <= norder <= 32. */
 int susy_b200_cg_freeze_iterations(susy_b200_lattice *h, int *iters, int norder);
-/* Solver launch mode (no reference counterpart): on = 1 captures the ~80
- * kernel launches of 16 solver iterations into a CUDA graph once per solve
- * and operator precision and replays it; on = 0 launches them one by one.
- * The default, reported as 1, leaves the choice to the solver (it launches
- * them, which is faster).  Same kernels, same results.  on < 0 only queries;
- * returns the previous setting. */
+/* Solver launch mode (no reference counterpart): on = 0 (default) launches
+ * the ~80 kernels of 16 solver iterations one by one, which is faster; on = 1
+ * captures them into a CUDA graph once per solve and operator precision and
+ * replays it.  Same kernels, same results.  on < 0 only queries; returns the
+ * previous setting. */
 int susy_b200_use_graphs(susy_b200_lattice *h, int on);
 /* Trajectory pseudofermion solves (no reference counterpart; the reference
  * solves them one after the other, update_o.c:98-113): on = 1 (default)

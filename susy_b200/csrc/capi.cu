@@ -264,7 +264,6 @@ susy_b200_lattice* solver_shadow(susy_b200_lattice* h) {
   c->G = h->G;
   c->ms_blocked = h->ms_blocked;
   c->use_graphs = h->use_graphs;
-  c->graphs_asked = h->graphs_asked;
   c->mix_switch = h->mix_switch;
   c->mix_reliable = h->mix_reliable;
   c->mix_interval = h->mix_interval;
@@ -457,7 +456,7 @@ int susy_b200_set_solver(susy_b200_lattice* h, int solver) {
 int susy_b200_use_graphs(susy_b200_lattice* h, int on) {
   if (!h) return SUSY_B200_EINVAL;
   const int prev = h->use_graphs;
-  if (on >= 0) h->use_graphs = h->graphs_asked = on ? 1 : 0;
+  if (on >= 0) h->use_graphs = on ? 1 : 0;
   return prev;
 }
 

@@ -45,9 +45,7 @@ struct susy_b200_lattice {
   double* meas = nullptr;     // measurement partials
   size_t meas_n = 0;
   int ms_blocked = 1;         // FP64 multi-shift CG: blocked vector update
-  int use_graphs = 1;         // susy_b200_use_graphs: 0 = never replay the solver's
-                              // iteration chunks as CUDA graphs
-  int graphs_asked = 0;       // replay them: set by an explicit use_graphs(1)
+  int use_graphs = 0;         // replay the solver's iteration chunks as CUDA graphs
   int host_solver = 0;        // solver behind susy_b200_congrad_multi
   double mix_switch = 3e-4;   // mixed solver: FP32 operator once |r| < this |src|
   double mix_reliable = 1e-2; // mixed solver: true residual when |r| fell this much

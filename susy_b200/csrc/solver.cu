@@ -483,18 +483,17 @@ static int ms_run_block(susy_b200_lattice* h, const void* src, void* const* psim
   };
   // fp32_below = 1: the FP32 operator from the first iteration
   if (mixed && h->mix_switch >= 1.0 && !to_fp32(0)) return set_err(h, SUSY_B200_ENOMEM);
-  // A caller that asked for graphs gets a chunk's ~80 launches captured once
-  // per operator precision and replayed: every argument of them is fixed for
-  // the solve (the convergence test and the freezing of shifts read device
-  // state).  Otherwise they are launched: programmatic dependent launches are
+  // With use_graphs a chunk's ~80 launches are captured once per operator
+  // precision and replayed: every argument of them is fixed for the solve (the
+  // convergence test and the freezing of shifts read device state).  By
+  // default they are launched: programmatic dependent launches are
   // issued faster than they run, and capturing and instantiating cost each
   // solve 0.2 to 0.4 ms (4^4 U(2) solve 2.92 ms with graphs, 2.71 without;
   // 4^4 trajectory 44.8 and 42.6, with two pseudofermions 58.8 and 52.0; 24
   // lattices' trajectories on 24 threads 503 and 451 ms).
-  const bool replay = h->use_graphs && h->graphs_asked;
   ChunkGraph graphs[2];
   for (;;) {
-    if (replay && h->use_graphs) {
+    if (h->use_graphs) {
       ChunkGraph& cg = graphs[fp32_op ? 1 : 0];
       if (!cg.ready) cg.capture(h, fp32_op ? 32 : 64, issue_chunk);
       if (cg.ready)

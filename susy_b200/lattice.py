@@ -513,8 +513,8 @@ class Lattice:
         return self._check(self.lib.susy_b200_set_solver(self.h, int(solver)))
 
     def use_graphs(self, on: int = -1) -> int:
-        """CUDA-graph replay (1) or plain launches (0) of the solver's
-        iteration chunks; returns the previous setting."""
+        """Plain launches (0, the default) or CUDA-graph replay (1) of the
+        solver's iteration chunks; returns the previous setting."""
         return self._check(self.lib.susy_b200_use_graphs(self.h, int(on)))
 
     def pf_streams(self, on: int = -1) -> int:

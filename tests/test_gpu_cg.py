@@ -99,6 +99,19 @@ def test_graph_replay_matches_plain_launches(mixed):
         assert np.array_equal(a, b)
 
 
+def test_graph_setting_round_trips():
+    """The setting reported is the one in force: a new handle launches and
+    says so, and saving a value, changing it and writing it back restores it."""
+    lat = Lattice((4, 4, 4, 4), 2, pbc=-1)
+    assert lat.use_graphs() == 0
+    for value in (0, 1):
+        lat.use_graphs(value)
+        saved = lat.use_graphs(1 - value)
+        assert saved == value and lat.use_graphs() == 1 - value
+        lat.use_graphs(saved)
+        assert lat.use_graphs() == value
+
+
 def test_microbench_operator_precisions_and_solvers():
     """The operator and solver microbenchmark configuration (8^4 U(2),
     links identity + 0.2 noise, lambda 1, bmass 0.2, G 0.05): D^dag D in
