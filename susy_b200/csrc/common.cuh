@@ -342,6 +342,8 @@ inline void launch_dep(void (*kernel)(P...), dim3 grid, dim3 block, cudaStream_t
   cfg.attrs = &at;
   cfg.numAttrs = 1;
   count_launch();
-  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  // no cast to the parameters' types: an argument that does not convert to
+  // its parameter by itself is refused, as <<<>>> refuses it
+  cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 }  // namespace susy

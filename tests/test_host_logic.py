@@ -168,3 +168,19 @@ def test_dependent_kernels_read_fields_with_ordinary_loads():
         assert "__ldg" not in src and not re.search(r"\bldc\s*<", src), name
         for call in re.findall(r"\b(?:ldm|ldtr|trace_ld)\s*<([^>]*)>", src):
             assert call.replace(" ", "").endswith(",true") and call.count(",") == 3, (name, call)
+
+
+@pytest.mark.parametrize("arg,compiles", [("double* q", True), ("float* q", False),
+                                          ("long q", False)])
+def test_dependent_launch_checks_its_arguments(tmp_path, arg, compiles):
+    """launch_dep refuses an argument that does not convert to the kernel's
+    parameter, as <<<>>> does (a functional cast would take any pointer)."""
+    import subprocess
+    from susy_b200 import build
+    src = tmp_path / "launch.cu"
+    src.write_text('#include "common.cuh"\n'
+                   "__global__ void k(const double*, long) { susy::wait_prior(); }\n"
+                   "void f(%s) { susy::launch_dep(k, 1, 32, (cudaStream_t)0, q, 3); }\n" % arg)
+    r = subprocess.run([build.nvcc(), "-c", str(src), "-o", str(tmp_path / "launch.o"),
+                        "-I" + build.CSRC, "-std=c++17"] + build.ARCH, capture_output=True)
+    assert (r.returncode == 0) == compiles, r.stderr.decode()[-2000:]
