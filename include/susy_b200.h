@@ -458,7 +458,10 @@ int susy_b200_DSq_batch(susy_b200_lattice *const *h, const void *const *src, voi
  * device; src[i] and psim[i][j] are FP64 device fields of h[i].  Launches on
  * cuda_stream (NULL: h[0]'s stream) after the work queued on every handle's
  * stream, and returns once the solves are done.  Uses each handle's solver
- * state and scratch fields.  Returns the largest iteration count or a
+ * state and scratch fields, norder[i] + 12 FP64 fields of lattice i in all,
+ * kept with the handle; where they do not fit the lattices are solved one
+ * after the other in the per-iteration form, which holds norder[i] + 4, each
+ * on its handle's stream.  Returns the largest iteration count or a
  * negative error code. */
 int susy_b200_dev_congrad_multi_batch(susy_b200_lattice *const *h, const void *const *src,
                                       void *const *const *psim, const int *norder,

@@ -268,10 +268,55 @@ static int ms_run_batch(susy_b200_lattice* const* hs, int nl, const void* const*
   return rc;
 }
 
+// Every field ms_run_batch takes of one handle
+static bool batch_fields(susy_b200_lattice* h, int norder) {
+  for (int which : {0, 3, 5})
+    if (!scratch_tf(h, which, 64)) return false;
+  return partials(h, 0) && partials(h, 1) && pvec(h, 0, norder, 64) &&
+         pvec(h, norder - 1, norder, 64) && ring_field(h, 0);
+}
+
+// The blocked update holds norder + 12 fields a lattice, the per-iteration one
+// norder + 4.  A batch of which only the latter fits is solved lattice by
+// lattice in that form, each on its own stream.
 int multishift_batch(susy_b200_lattice* const* hs, int nl, const void* const* src,
                      void* const* const* psim, const int* norder, const double* const* shift,
                      int MaxCG, double errormin, double* size_r, int* iters, cudaStream_t st) {
-  return ms_run_batch(hs, nl, src, psim, norder, shift, MaxCG, errormin, size_r, iters, st);
+  std::vector<int> err(nl);
+  std::vector<char> had_ring(nl);
+  bool fits = true;
+  for (int i = 0; i < nl; i++) {
+    err[i] = hs[i]->err;
+    had_ring[i] = !hs[i]->ring.empty();
+  }
+  for (int i = 0; i < nl && fits; i++) fits = batch_fields(hs[i], norder[i]);
+  if (fits)
+    return ms_run_batch(hs, nl, src, psim, norder, shift, MaxCG, errormin, size_r, iters, st);
+  for (int i = 0; i < nl; i++) {
+    susy_b200_lattice* h = hs[i];
+    h->err = err[i];
+    if (had_ring[i] || h->ring.empty()) continue;
+    cudaFree(h->ring[0]);   // the ring is one allocation (family)
+    h->extra.erase(std::find(h->extra.begin(), h->extra.end(), h->ring[0]));
+    h->ring.clear();
+  }
+  if (cudaStreamSynchronize(st) != cudaSuccess) return SUSY_B200_ECUDA;
+  for (int i = 0; i < nl; i++) {
+    susy_b200_lattice* h = hs[i];
+    double rsq = 0.0;
+    int it = 0;
+    // the batched operator's kernel where none is tuned: tuning takes two
+    // more fields
+    const int variant = h->fop_variant[0];
+    if (variant < 0) h->fop_variant[0] = FOP_ROLLING;
+    const int rc = ms_run(h, src[i], psim[i], norder[i], shift[i], MaxCG, errormin, 64, 64,
+                          &rsq, &it);
+    h->fop_variant[0] = variant;
+    if (rc < 0) return rc;
+    if (size_r) size_r[i] = rsq;
+    if (iters) iters[i] = it;
+  }
+  return SUSY_B200_OK;
 }
 
 // FP32 residual ring slots 0..MS_BLK of the mixed solver's FP32 phase

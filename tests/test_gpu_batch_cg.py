@@ -124,3 +124,43 @@ def test_batch_solve_waits_for_each_handles_own_stream(cuda_stream):
             res = true_residuals(lat, srcs[k].download(), psims[k], shifts, fm)
             assert max(res) <= 1e-18, (rnd, k, res)
             lat.fop_variant(64, 10)
+
+
+def test_batch_solve_where_only_the_smaller_workspace_fits():
+    """Device memory left for the per-iteration solve's norder + 4 fields of
+    each lattice but not for the blocked one's norder + 12: the batch is
+    still solved, with the solo iteration count, leaves no error behind, and
+    gives the residual ring back.  Residual bound as above."""
+    import torch
+    dims, shifts = (16, 16, 16, 16), synth.geometric_shifts(3, 1e-2, 1.0)
+    rng = np.random.default_rng(5)
+    lats, srcs, psims = [], [], []
+    for k in range(2):
+        lat = Lattice(dims, 2, pbc=-1, lam=1.0, bmass=0.2, G=0.05)
+        lat.set_links(synth.to_ref(dims, synth.links(dims, 2, 0.2, 60 + k)))
+        src = lat.tf(64)
+        src.upload(rng.standard_normal(lat.tf_doubles))
+        lats.append(lat)
+        srcs.append(src)
+        psims.append([lat.tf(64) for _ in shifts])
+    field = 16 * 4 * 16 ** 4 * 16
+    need_small, need_large = 2 * (len(shifts) + 4) * field, 2 * (len(shifts) + 12) * field
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    hold = torch.empty(free - (need_small + need_large) // 2, dtype=torch.uint8, device="cuda")
+    left = torch.cuda.mem_get_info()[0]
+    assert need_small + 2 * field < left < need_large - 2 * field
+    try:
+        iters, rsq = congrad_multi_batch(srcs, psims, [shifts] * 2, 5000, 1e-20)
+        used = left - torch.cuda.mem_get_info()[0]
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    assert used < need_small + 2 * field
+    for k, lat in enumerate(lats):
+        assert lat.lib.susy_b200_last_error(lat.h) == 0
+        res = true_residuals(lat, srcs[k].download(), psims[k], shifts, 0.0)
+        assert max(res) <= 1e-18 and np.isfinite(rsq[k]), res
+        lat.cg_blocked(0)
+        it, _ = lat.dev_congrad_multi(srcs[k], psims[k], shifts, 5000, 1e-20)
+        assert abs(it - iters[k]) <= 1
