@@ -153,6 +153,11 @@ int autotune_fop(susy_b200_lattice* h, int prec) {
   float best = 1e30f;
   int bestv = h->rescale ? FOP_SITE_MAJOR_OCC : FOP_MAT;
   for (int v = h->rescale ? FOP_COMPACT : 0; v < FOP_NVARIANTS; v++) {
+    // the same launch as FOP_ROLLING for NCOL 4 (fermion_op_rolling)
+    if (v == FOP_ROLLING_WIDE && h->N == 4) {
+      h->fop_ms[pi][v] = h->fop_ms[pi][FOP_ROLLING];
+      continue;
+    }
     launch_variant(h, a, b, 1, prec, nullptr, 0.0, nullptr, nullptr, v, FOP_ALONE);
     cudaEventRecord(e0, h->stream);
     for (int r = 0; r < 3; r++) {
