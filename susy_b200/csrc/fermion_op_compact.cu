@@ -61,7 +61,9 @@ int upload_fop_terms(int device, cudaStream_t st) {
   cudaMemcpyToSymbol(c_pat_start, start, sizeof(start));
   cudaMemcpyToSymbol(c_disp, tb.disp.data(), tb.disp.size() * sizeof(char4));
   if (upload_force_terms() != 0 || upload_rolling_terms() != 0) return -2;
-  if (cudaGetLastError() != cudaSuccess) return -2;
+  // small copies return before they land, and a handle's stream does not wait
+  // for the default stream they went to
+  if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) return -2;
   prefer_l1_grouped<double>();
   prefer_l1_grouped<float>();
   if (device >= 0 && device < 64) g_terms_ready[device] = true;
