@@ -820,9 +820,9 @@ def run_batch_cg_case(args):
     """The multi-shift solve (15 shift4 poles of the Nroot 1 degree-15
     approximation, FP64 residual 1e-10 per site) on --lattices independent
     U(2) lattices of the batched scan: all lattices in one batched solve
-    (susy_b200_dev_congrad_multi_batch: six launches per iteration for all
+    (susy_b200_dev_congrad_multi_batch: five launches per iteration for all
     of them) against each lattice's own solve in turn (its default FP64
-    solver: blocked vector update, graph-replayed iteration chunks), every
+    solver, the same blocked vector update), every
     lattice on one stream.  Device time with CUDA events; also the largest
     iteration difference and the largest relative solution difference."""
     import torch

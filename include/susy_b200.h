@@ -430,28 +430,30 @@ int susy_b200_update_batch(susy_b200_lattice *const *h, const susy_b200_rhmc *co
 
 /* dst[i] = (D^dag D + fmass_i^2) src[i] on lattice h[i], for n independent
  * lattices in two persistent launches over one work table of (lattice,
- * 128-site tile, output component) items instead of two launches per
- * lattice (no reference counterpart: the reference applies DSq,
+ * 128-site tile, output component) items, after one launch for the
+ * determinant traces of every lattice with G > 0, instead of two or three
+ * launches per lattice (no reference counterpart: the reference applies DSq,
  * utilities.c:874, to one lattice per process).  1 <= n <= 64 handles of
  * one NCOL on one device; lattice sizes, couplings and the RESCALE setting
  * may differ.  src[i] and dst[i] are device fields of h[i] in precision
  * prec (64 or 32).  Launches on cuda_stream (NULL: h[0]'s stream), after
  * the work already queued on every handle's stream, which in turn waits
  * for the launches, so the call is ordered like each handle's own
- * susy_b200_dev_DSq.  Each lattice's result is the one the site-major
- * table-driven kernels give it alone.  Uses (and on first use allocates)
+ * susy_b200_dev_DSq.  Each lattice's result is the one the rolling kernels
+ * (operator variants 10 and 11) give it alone.  Uses (and on first use allocates)
  * each handle's DSq scratch field. */
 #define SUSY_B200_BATCH_MAX 64
 int susy_b200_DSq_batch(susy_b200_lattice *const *h, const void *const *src, void *const *dst,
                         int n, int prec, void *cuda_stream);
 /* congrad_multi (susy/congrad_multi.c:26) for n independent lattices at
- * once, FP64, the reference's recurrences in their per-iteration form (the
- * solve susy_b200_cg_blocked(h, 0) selects for one lattice): lattice i
+ * once, FP64, the reference's recurrences with the blocked vector update (the
+ * default solve of one lattice, whatever susy_b200_cg_blocked says): lattice i
  * solves (D^dag D + fmass_i^2 + shift[i][j]) psim[i][j] = src[i] for
- * j < norder[i], each iteration being six launches for all lattices (the
+ * j < norder[i], each iteration being five launches for all lattices (the
  * batched operator of susy_b200_DSq_batch, D^dag with the dot product in its
- * epilogue, the recurrences one block per lattice, the vector updates over
- * one table of blocks).  Each lattice stops at its own iteration, as it
+ * epilogue, the first recurrences one block per lattice, the residual update
+ * with the second ones and the p0 update over tables of blocks) and every
+ * eighth a pass over the live shifts' vectors.  Each lattice stops at its own iteration, as it
  * would alone; size_r[i] and iters[i] (either may be NULL) receive its final
  * |r|^2 and iterations.  No counterpart in the reference, which solves one
  * lattice per process.  1 <= n <= 64 distinct handles of one NCOL on one

@@ -334,10 +334,13 @@ template void fop_traces<double>(const Geo&, int, const void*, const void*, void
 template void fop_traces<float>(const Geo&, int, const void*, const void*, void*, cudaStream_t);
 
 // Resident blocks per SM: as many as hold a product's operands, the
-// accumulator and the addresses without spilling (80 / 64 registers for
-// NCOL 2, 128 / 80 for 3, 255 / 128 for 4, FP64 / FP32).  wide: a step fewer,
-// for lattices that do not fill the GPU anyway: more loads hoisted
-// (6^3x12 U(3) FP64 39.2 against 41.9 us; 12^3x24 293 against 263).
+// accumulator and the addresses (80 / 64 registers for NCOL 2, 128 / 80 for 3,
+// 255 / 128 for 4, FP64 / FP32) with at most 32 bytes spilled a thread (ptxas:
+// 32 in the FP64 D^dag of NCOL 3, 8 or 16 in the FP32 kernels of NCOL 3, 4 in
+// the wide FP64 ones of NCOL 2; a spilled operand waits for its load, and a
+// form that spilled many took twice the time).  wide: a step fewer, for
+// lattices that do not fill the GPU anyway: more loads hoisted (D^dag D of 6^3x12 U(3) FP64 32.0 against 33.1 us,
+// 12^3x24 257.7 against 244.1).
 template <typename R>
 int fermion_op_rolling(const FopArgs<R>& a, int N, int sign, bool wide, cudaStream_t st) {
   constexpr bool D = sizeof(R) == 8;

@@ -110,7 +110,7 @@ int upload_force_terms() {
 //   tr[6 + e] = Tr U_e^-1 psi'_e^dag, tr[11] = conj Tr eta'
 // (psi, eta of sol, primed of psol).  The rolling operator kernels leave
 // exactly these in their trace field when they form psol = D sol; this
-// pre-pass (19 us a pole at 12^3x24 U(3)) serves the other kernels.  One thread
+// pre-pass (21 us a pole at 12^3x24 U(3)) serves the other kernels.  One thread
 // per site and e = blockIdx.y; e = 5 the two of the site component.
 template <int N>
 __global__ void __launch_bounds__(FT) k_ff_traces(FfArgs a, double2* tr) {
@@ -205,7 +205,7 @@ SUSY_D void ff_pattern(Mat<N, double>& acc, const FfArgs& a, int s, unsigned bcm
 // loop so that a thread holds two operands and an accumulator: the kernel
 // this replaces unrolled all 44 products and 80 traces per link and lived in
 // local memory (per thread 8 KB of stack for NCOL 3, 45 KB for NCOL 4).
-// 12^3x24 U(3): 199 us a pole and 19 us of traces, against 1359 us.
+// 12^3x24 U(3): 203 us a pole and 21 us of traces, against 1359 us.
 template <int N>
 constexpr int ff_blocks() { return N == 2 ? 6 : (N == 3 ? 4 : 2); }
 

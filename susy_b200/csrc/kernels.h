@@ -95,8 +95,9 @@ struct MsBlockVecs {
 // FOP_ROLLING / FOP_ROLLING_WIDE: table-driven by link direction, each
 // product's operands loaded while the one before it computes, the
 // determinant terms from the trace pre-pass (fermion_op_rolling.cu; without
-// the trace field they run as FOP_SITE_MAJOR_FRONT).  The autotuner's pick
-// from 8^4 on.
+// the trace field they run as FOP_SITE_MAJOR_FRONT).  One of the two is the
+// autotuner's pick on every lattice timed, 4^4 U(2) (16.6 us a D^dag D against
+// 25.6 for the best other) to 24^4 U(2) (872 against 1350).
 // FOP_SITE_MAJOR_FRONT: site-major (FP64 4, FP32 8 blocks per SM) with the
 // site component's long blocks at the front of the grid.
 // FOP_GROUPED: one output component per warp over the same 32 sites, the

@@ -586,7 +586,8 @@ def update_batch(lattices, rhmcs, threads: int = 8):
 
 def dsq_batch(srcs, dsts, stream_ptr: int | None = None):
     """dst[i] = (D^dag D + fmass^2) src[i] on each DeviceTF's lattice, all
-    lattices in two launches (susy_b200_DSq_batch); one NCOL and precision."""
+    lattices in two launches and one for their determinant traces
+    (susy_b200_DSq_batch); one NCOL and precision."""
     n = len(srcs)
     assert len(dsts) == n and n > 0
     lats = [s.lat for s in srcs]

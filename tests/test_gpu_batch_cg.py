@@ -1,11 +1,11 @@
 """congrad_multi on many lattices at once (susy_b200_dev_congrad_multi_batch).
 
 Every lattice of the batch must follow its own solve: the same FP64
-recurrences as the per-iteration solver run alone (susy_b200_cg_blocked(h,
-0)), so its iteration count within 1 of the solo one and every shift's
+recurrences (with the blocked vector update) as the per-iteration solver run
+alone (susy_b200_cg_blocked(h, 0)), so its iteration count within 1 of the solo one and every shift's
 solution within 1e-8 relative (max-norm) of the solo solution at an FP64
-residual of 1e-10 per site (the two differ only in the summation order of
-the inner products).  The lattices differ in extents, couplings, fermion
+residual of 1e-10 per site (the two differ in the operator kernel, the vector
+update's form and the summation order of the inner products).  The lattices differ in extents, couplings, fermion
 mass, boundary condition, RESCALE and their shifts, so they stop at
 different iterations while the others go on.
 """
@@ -16,7 +16,7 @@ from susy_b200 import Lattice, SusyError, congrad_multi_batch, synth
 
 pytestmark = pytest.mark.gpu
 
-FRONT = 12   # FOP_SITE_MAJOR_FRONT: the batched operator's products and order
+FRONT = 12   # FOP_SITE_MAJOR_FRONT: an operator kernel that reads no traces
 
 CASES = [  # dims, lambda, G, fmass, pbc, rescale, shifts
     ((4, 4, 4, 4), 1.0, 0.05, 0.0, -1, 0, synth.geometric_shifts(6, 1e-3, 1.0)),

@@ -2,10 +2,11 @@
 
 The batched D^dag D walks one work table of (lattice, 128-site tile, output
 component) items for all lattices in a single persistent launch per sign.
-Each lattice must get what its own site-major table-driven kernel gives it
-(variant FOP_SITE_MAJOR_FRONT, the same products in the same order): FP64
-within 1e-13 and FP32 within 1e-6 relative (max-norm), and the FP64 result
-of one lattice is also checked against the numpy oracle at 1e-13.
+Its items are the rolling kernels' blocks; each lattice must get what a kernel
+of another design gives it alone (variant FOP_SITE_MAJOR_FRONT: the same
+products in another order, the traces formed where they are used): FP64
+within 1e-13 and FP32 within 1e-6 relative (max-norm), and the FP64 result of
+one lattice is also checked against the numpy oracle at 1e-13.
 Lattices differ in extents, couplings (G = 0 switches the determinant
 terms off), fermion mass, boundary condition and the RESCALE setting.
 """
