@@ -339,8 +339,8 @@ template void fop_traces<float>(const Geo&, int, const void*, const void*, void*
 // 32 in the FP64 D^dag of NCOL 3, 8 or 16 in the FP32 kernels of NCOL 3, 4 in
 // the wide FP64 ones of NCOL 2; a spilled operand waits for its load, and a
 // form that spilled many took twice the time).  wide: a step fewer, for
-// lattices that do not fill the GPU anyway: more loads hoisted (D^dag D of 6^3x12 U(3) FP64 32.0 against 33.1 us,
-// 12^3x24 257.7 against 244.1).
+// lattices that do not fill the GPU anyway: more loads hoisted (D^dag D of
+// 6^3x12 U(3) FP64 32.0 against 33.1 us, 12^3x24 257.7 against 244.1).
 template <typename R>
 int fermion_op_rolling(const FopArgs<R>& a, int N, int sign, bool wide, cudaStream_t st) {
   constexpr bool D = sizeof(R) == 8;
