@@ -876,8 +876,11 @@ __global__ void __launch_bounds__(UT, 6) k_msbat_update_r(const MsLat* L, int nl
   update_r_block<double2, double2>(l.st, l.v, l.n, l.part1, blockIdx.x - l.rblk0, l.rblocks);
 }
 
+// Blocks per SM: 40, 64 and 128 registers for NCOL 2, 3 and 4 (left to itself
+// the compiler takes 48 for NCOL 2: the 12-lattice solve 69.2-69.3 ms, 68.6-68.9
+// with the bound)
 template <int N>
-__global__ void __launch_bounds__(UT) k_msbat_update_p0(const MsLat* L, int nl) {
+__global__ void __launch_bounds__(UT, N == 2 ? 6 : (N == 3 ? 4 : 2)) k_msbat_update_p0(const MsLat* L, int nl) {
   wait_prior();
   const MsLat& l = L[vblock_lattice<&MsLat::qblk0>(L, nl, blockIdx.x)];
   msb_p0_block<N, double2, double>(l.st, l.v, blockIdx.x - l.qblk0);
