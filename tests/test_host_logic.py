@@ -131,7 +131,7 @@ def _dependent_code():
         if not f.endswith((".cu", ".cuh")):
             continue
         src = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, f)).read())
-        src = re.sub(r"__launch_bounds__\((?:[^()]|\(\))*\)", "", src)
+        src = re.sub(r"__launch_bounds__\((?:[^()]|\([^()]*\))*\)", "", src)
         launched |= set(re.findall(r"launch_dep\(\s*(\w+)", src)) - {"void"}
         for m in re.finditer(r"(?:SUSY_D|__global__)[^;{}=]*?(\w+)\s*\([^;{}]*\)\s*\{", src):
             depth, i = 1, m.end()
